@@ -30,8 +30,10 @@ __device__ __forceinline__ vec3<TF> rotate(vec3<TF> v, vec4<TF> q) {
 template <class TF>
 __device__ __forceinline__ TF box_sdf(vec3<TF> x, TF hx, TF hy, TF hz, TF outset) {
   vec3<TF> d{fabs(x.x) - hx, fabs(x.y) - hy, fabs(x.z) - hz};
+  const TF m = fmax(d.x, fmax(d.y, d.z));
+  if (m <= TF(0)) return m - outset;  // inside: no square root
   vec3<TF> cl{fmax(d.x, TF(0)), fmax(d.y, TF(0)), fmax(d.z, TF(0))};
-  return sqrt(length_sqr(cl)) + fmin(fmax(d.x, fmax(d.y, d.z)), TF(0)) - outset;
+  return sqrt(length_sqr(cl)) - outset;
 }
 
 // Analytic signed distances (dg/box_distance.hpp:23-30,

@@ -13,13 +13,13 @@ namespace {
 inline uint32_t blocks_for(uint32_t n, int block) { return (n + block - 1) / block; }
 
 // Quadrature tables in constant memory: per azimuth i cos/sin(theta_i), per
-// polar node j sin/cos(phi_j), per (j, k) the weight 2 pi b_j c_k / 60, per
-// k the radius.
+// polar node j sin/cos(phi_j), per (j, k) the weight 2 pi b_j c_k / 60 as the
+// double it is summed with, per k the radius.
 template <class T>
 struct PeirceTab {
   T ct[peirce::kNumTheta], st[peirce::kNumTheta];
   T sp[peirce::kNumPhi], cp[peirce::kNumPhi];
-  T w[peirce::kNumPhi * peirce::kNumR];
+  double wd[peirce::kNumPhi * peirce::kNumR];  // the weights rounded to T
   T r[peirce::kNumR];
 };
 using PeirceDev = PeirceTab<float>;
@@ -198,37 +198,101 @@ __global__ void k_distance_grid(BodyDev<TF> b, TF* __restrict__ out) {
   out[l] = shape_sdf(b, node_position(b, l));
 }
 
-// update_volume_field: one warp per node; lanes stride over the 27,000
-// (theta, phi, r) samples and accumulate in double; the warp sum is the
-// node's integral times h^3.
+// Distance below which every sample of a node's ball lies inside the body
+// and above which every sample is farther than h from it.  The samples are
+// less than h away from the node and the analytic distances are 1-Lipschitz,
+// so a signed distance above 2 h means a distance above h at every sample
+// (integrand 0) and one below -h a negative distance at every sample
+// (integrand 1); the slack covers the rounding of the distances, which grows
+// with the coordinates and the shape's extents.
 template <class TF>
+__device__ __forceinline__ TF band_slack(const Cn<TF>& c, const BodyDev<TF>& b, vec3<TF> x) {
+  TF m = fmax(fabs(x.x), fmax(fabs(x.y), fabs(x.z)));
+#pragma unroll
+  for (int k = 0; k < 8; ++k) m = fmax(m, fabs(b.p[k]));
+  return c.h * TF(1e-3) + m * (sizeof(TF) == 4 ? TF(4e-6) : TF(8e-15));
+}
+
+// The integrand of the volume map at signed distance dm: 1 inside, W(dm) /
+// W(0) outside (dist_cubic_kernel with 1 / h and k / W(0) rounded once).
+template <class TF>
+__device__ __forceinline__ TF extension(TF dm, TF inv_h, TF k_w0) {
+  if (dm <= TF(0)) return TF(1);
+  const TF q = dm * inv_h, conj = TF(1) - q;
+  const TF s = q <= TF(0.5) ? (TF(6) * q - TF(6)) * q * q + TF(1)
+                            : (q <= TF(1) ? TF(2) * conj * conj * conj : TF(0));
+  return s * k_w0;
+}
+
+// What k_volume_field takes distances from: the body's grid, or its analytic
+// shape, either read from the body or fixed at compile time.
+constexpr int kFromGrid = -2, kAnyShape = -1;
+
+// update_volume_field: one warp per node over the 60 x 30 x 15 (theta, phi,
+// r) samples.  Lane l takes the azimuths l and l + 32 (registers); the polar
+// and radial loops are uniform, so their tables are broadcast constant reads
+// (a flat sample index per lane cost two integer divisions and up to 32
+// different constant addresses per read).  The integrand is summed in
+// double.  Analytic shapes skip the nodes whose ball misses the band -h ..
+// 2 h around the surface, which are constants (`full` = the sum of the
+// weights); the shapes of walls and balls are compiled apart, so that no
+// sample branches on the shape.  Measured (B200, container box, 32^3 cells,
+// 217,800 nodes, 53 % of them in the band): 93.3 ms with flat sample indices
+// over all nodes, 8.2 ms now.
+template <class TF, int FROM>
 __global__ void __launch_bounds__(256)
-    k_volume_field(Cn<TF> c, BodyDev<TF> b, TF* __restrict__ out) {
+    k_volume_field(Cn<TF> c, BodyDev<TF> b, double full, TF* __restrict__ out) {
+  if constexpr (FROM >= 0) b.shape = uint32_t(FROM);
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= b.num_nodes) return;
   const auto& pt = PeirceSel<TF>::get();
   const vec3<TF> x = node_position(b, warp);
-  constexpr int kDirs = peirce::kNumTheta * peirce::kNumPhi;
+  const double h3 = double(c.h2) * double(c.h);
+  if constexpr (FROM != kFromGrid) {
+    const TF phi = shape_sdf(b, x) * b.sign;
+    const TF slack = band_slack(c, b, x);
+    const bool outside = phi > TF(2) * c.h + slack;
+    if (outside || phi < -(c.h + slack)) {
+      if (lane == 0) out[warp] = outside ? TF(0) : TF(full * h3);
+      return;
+    }
+  }
+  const TF k_w0 = c.k / c.w0;
+  const bool second = lane + 32 < peirce::kNumTheta;
+  const int i1 = second ? lane + 32 : lane;
+  const TF ct[2] = {pt.ct[lane], pt.ct[i1]}, st[2] = {pt.st[lane], pt.st[i1]};
   double sum = 0;
-  for (int f = lane; f < kDirs * peirce::kNumR; f += 32) {
-    const int k = f % peirce::kNumR;
-    const int dir = f / peirce::kNumR;  // dir = i * kNumPhi + j
-    const int j = dir % peirce::kNumPhi;
-    const int i = dir / peirce::kNumPhi;
-    const TF rr = c.h * pt.r[k];
-    const TF ux = pt.sp[j] * pt.ct[i], uy = pt.sp[j] * pt.st[i], uz = pt.cp[j];
-    const vec3<TF> p{x.x + rr * ux, x.y + rr * uy, x.z + rr * uz};
-    const TF dist = b.use_grid ? interpolate_grid(b, b.dist, p) : shape_sdf(b, p);
-    const TF dm = dist * b.sign;
-    const TF ext = dm <= TF(0) ? TF(1) : W_dist(c, dm) / c.w0;
-    sum += double(pt.w[j * peirce::kNumR + k]) * double(ext);
+  for (int j = 0; j < peirce::kNumPhi; ++j) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      if (e && !second) break;
+      const TF ux = pt.sp[j] * ct[e], uy = pt.sp[j] * st[e], uz = pt.cp[j];
+#pragma unroll
+      for (int k = 0; k < peirce::kNumR; ++k) {
+        const TF rr = c.h * pt.r[k];
+        const vec3<TF> p{x.x + rr * ux, x.y + rr * uy, x.z + rr * uz};
+        TF dist;
+        if constexpr (FROM == kFromGrid)
+          dist = interpolate_grid(b, b.dist, p);
+        else
+          dist = shape_sdf(b, p);
+        sum += pt.wd[j * peirce::kNumR + k] * double(extension(dist * b.sign, c.inv_h, k_w0));
+      }
+    }
   }
   sum = warp_sum(sum);
-  if (lane == 0) out[warp] = TF(sum * double(c.h2) * double(c.h));
+  if (lane == 0) out[warp] = TF(sum * h3);
 }
 
 }  // namespace
+
+// Weight of a (phi_j, r_k) sample, rounded to TF.
+template <class TF>
+double peirce_weight(int j, int k) {
+  const double pi = 3.14159265358979323846264338327950288;
+  return double(TF(2 * pi * peirce::k_b[j] * peirce::k_c[k] / peirce::kNumTheta));
+}
 
 int upload_peirce_tables(cudaStream_t st) {
   static PeirceDev tf;
@@ -249,9 +313,8 @@ int upload_peirce_tables(cudaStream_t st) {
   }
   for (int j = 0; j < peirce::kNumPhi; ++j)
     for (int k = 0; k < peirce::kNumR; ++k) {
-      td.w[j * peirce::kNumR + k] =
-          2 * pi * peirce::k_b[j] * peirce::k_c[k] / peirce::kNumTheta;
-      tf.w[j * peirce::kNumR + k] = float(td.w[j * peirce::kNumR + k]);
+      td.wd[j * peirce::kNumR + k] = peirce_weight<double>(j, k);
+      tf.wd[j * peirce::kNumR + k] = peirce_weight<float>(j, k);
     }
   for (int k = 0; k < peirce::kNumR; ++k) {
     td.r[k] = peirce::k_r[k];
@@ -291,7 +354,20 @@ int sample_boundaries_fused(const Cn<TF>& c, const vec4<TF>* xs, uint32_t stride
 template <class TF>
 int build_volume_field(const Cn<TF>& c, const BodyDev<TF>& b, TF* out, cudaStream_t st) {
   const uint64_t threads = uint64_t(b.num_nodes) * 32;
-  k_volume_field<TF><<<uint32_t((threads + 255) / 256), 256, 0, st>>>(c, b, out);
+  const uint32_t blocks = uint32_t((threads + 255) / 256);
+  // the integral of 1: every sample inside
+  double full = 0;
+  for (int j = 0; j < peirce::kNumPhi; ++j)
+    for (int k = 0; k < peirce::kNumR; ++k)
+      full += peirce::kNumTheta * peirce_weight<TF>(j, k);
+  auto kernel = k_volume_field<TF, kAnyShape>;
+  if (b.use_grid)
+    kernel = k_volume_field<TF, kFromGrid>;
+  else if (b.shape == AL_SHAPE_BOX)
+    kernel = k_volume_field<TF, AL_SHAPE_BOX>;
+  else if (b.shape == AL_SHAPE_SPHERE)
+    kernel = k_volume_field<TF, AL_SHAPE_SPHERE>;
+  kernel<<<blocks, 256, 0, st>>>(c, b, full, out);
   ALB_CUDA(cudaGetLastError());
   return AL_OK;
 }
