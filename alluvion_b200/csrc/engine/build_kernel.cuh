@@ -108,6 +108,9 @@ __global__ void __launch_bounds__(kMaxBlock)
   const int z0 = max(ip[2] - 1, 0);
   const int z1 = min(ip[2] + 1, int(g.res[2]) - 1);
   uint32_t cnt = 0;
+  // the list's open group, newest entry last, written when it is full
+  uint4* list = reinterpret_cast<uint4*>(nbr) + s;
+  uint4 grp{s, s, s, s};
   // ---- phase 1: candidates -> list
   if (z0 <= z1) {
     for (int dx = -1; dx <= 1; ++dx) {
@@ -147,8 +150,10 @@ __global__ void __launch_bounds__(kMaxBlock)
           if (m < 32) acc &= (1u << m) - 1u;
           if (s - t0 < m) acc &= ~(1u << (s - t0));  // the particle itself
           for (; acc; acc &= acc - 1) {
-            if (cnt < g.cap_nbr)
-              nbr[size_t(cnt) * stride + s] = t0 + uint32_t(__ffs(acc) - 1);
+            if (cnt < g.cap_nbr) {
+              grp = uint4{grp.y, grp.z, grp.w, t0 + uint32_t(__ffs(acc) - 1)};
+              if (cnt % kNbrGroup == kNbrGroup - 1) list[size_t(cnt / kNbrGroup) * stride] = grp;
+            }
             ++cnt;
           }
         }
@@ -160,37 +165,42 @@ __global__ void __launch_bounds__(kMaxBlock)
     cnt = g.cap_nbr;
   }
   ncount[s] = cnt;
+  if (cnt % kNbrGroup) {  // the last group, padded with the particle itself
+    for (uint32_t k = cnt % kNbrGroup; k < kNbrGroup; ++k) grp = uint4{grp.y, grp.z, grp.w, s};
+    list[size_t(cnt / kNbrGroup) * stride] = grp;
+  }
   // ---- phase 2: density (+ factor, + EX) over the list, in list order
   TF density = c.vol * c.w0;
   TF sum_grad = 0;
   vec3<TF> grad_i{0, 0, 0};
   TF div = 0;
   const vec3<TF> vi = ex.self_v(s);
-  // list entries per round (measured on B200 with the 256-bit record loads,
-  // per build at 1,048,576 / 8,388,608 particles: 0.334 / 2.66 ms at 2,
-  // 0.338 / 2.71 at 4, 0.367 / 2.90 at 8)
+  // Two entries' records in flight at a time (with entries read one by one,
+  // per build at 1,048,576 / 8,388,608 particles: 0.334 / 2.66 ms at 2, 0.338
+  // / 2.71 at 4, 0.367 / 2.90 at 8).
   constexpr uint32_t kB = 2;
-  for (uint32_t k0 = 0; k0 < cnt; k0 += kB) {
-    uint32_t t[kB];
+  for (uint32_t g0 = 0; g0 < cnt; g0 += kNbrGroup) {
+    const uint4 q4 = list[size_t(g0 / kNbrGroup) * stride];  // this thread's own store
+    const uint32_t t[kNbrGroup] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
-    for (uint32_t q = 0; q < kB; ++q)  // this thread's own stores: plain loads
-      t[q] = k0 + q < cnt ? nbr[size_t(k0 + q) * stride + s] : s;
-    vec3<TF> xj[kB], vj[kB];
+    for (uint32_t h = 0; h < kNbrGroup; h += kB) {
+      vec3<TF> xj[kB], vj[kB];
 #pragma unroll
-    for (uint32_t q = 0; q < kB; ++q) ex.xv(xs, t[q], xj[q], vj[q]);
+      for (uint32_t q = 0; q < kB; ++q) ex.xv(xs, t[h + q], xj[q], vj[q]);
 #pragma unroll
-    for (uint32_t q = 0; q < kB; ++q) {
-      if (k0 + q >= cnt) break;
-      density += c.vol * W_r2(c, pdist2(c, xi, xj[q]));
-      if (FACTOR || EX::kOn) {
-        const vec3<TF> d = pdisp(c, xi, xj[q]);
-        const vec3<TF> gw = gradW(c, d);
-        if (FACTOR) {
-          const vec3<TF> gpj = (-c.vol) * gw;
-          sum_grad += length_sqr(gpj);
-          grad_i -= gpj;
+      for (uint32_t q = 0; q < kB; ++q) {
+        if (g0 + h + q >= cnt) break;
+        density += c.vol * W_r2(c, pdist2(c, xi, xj[q]));
+        if (FACTOR || EX::kOn) {
+          const vec3<TF> d = pdisp(c, xi, xj[q]);
+          const vec3<TF> gw = gradW(c, d);
+          if (FACTOR) {
+            const vec3<TF> gpj = (-c.vol) * gw;
+            sum_grad += length_sqr(gpj);
+            grad_i -= gpj;
+          }
+          if (EX::kOn) div += c.vol * dot(vi - vj[q], gw);
         }
-        if (EX::kOn) div += c.vol * dot(vi - vj[q], gw);
       }
     }
   }

@@ -384,7 +384,7 @@ int update_neighbors_impl(al_engine* e, const C* cn, const al_consti* cni, const
   TF* rho = nullptr;
   ALB_TRY(e->buf("sorted.x", size_t(n) + kSortedPad, &xs));
   ALB_TRY(e->buf("flags", 4, &flags));
-  ALB_TRY(e->buf("nbr.list", size_t(n) * g.cap_nbr, &nbr));
+  ALB_TRY(e->buf("nbr.list", nbr_list_words(n, g.cap_nbr), &nbr));
   ALB_TRY(e->buf("nbr.count", n, &ncount));
   ALB_TRY(e->buf("sorted.rho", n, &rho));
   ALB_CUDA(cudaMemsetAsync(flags, 0, 4 * sizeof(uint32_t), st));

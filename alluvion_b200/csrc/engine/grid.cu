@@ -239,13 +239,12 @@ inline uint32_t crowded_blocks(uint32_t ncells) {
 
 template <class TF>
 __global__ void k_gather_x(const TF* __restrict__ x, const uint32_t* __restrict__ perm,
-                           uint32_t n, vec4<TF>* __restrict__ xs, uint32_t* __restrict__ inv) {
+                           uint32_t n, vec4<TF>* __restrict__ xs) {
   uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   uint32_t i = perm[s];
   vec3<TF> p = ld3(x, i);
   xs[s] = vec4<TF>{p.x, p.y, p.z, TF(0)};
-  inv[i] = s;
 }
 
 inline uint32_t blocks_for(uint32_t n, int block) { return (n + block - 1) / block; }
@@ -327,7 +326,6 @@ int grid_build(al_engine* e, const Cn<TF>& c, const GridDims& g, const TF* parti
   ALB_TRY(e->buf("grid.cell", n, &gs.cell));
   ALB_TRY(e->buf("grid.rank", n, &rank));
   ALB_TRY(e->buf("grid.perm", n, &gs.perm));
-  ALB_TRY(e->buf("grid.inv", n, &gs.inv));
   ALB_TRY(e->buf("grid.count", size_t(g.ncells) + 1, &gs.count));
   ALB_TRY(e->buf("grid.start", size_t(g.ncells) + 2, &gs.cell_start));
   ALB_CUDA(cudaMemsetAsync(gs.count, 0, (size_t(g.ncells) + 1) * sizeof(uint32_t), st));
@@ -345,7 +343,7 @@ int grid_build(al_engine* e, const Cn<TF>& c, const GridDims& g, const TF* parti
                                                                  gs.perm);
   k_order_crowded<<<crowded_blocks(g.ncells), kCrowdedThreads, 0, st>>>(gs.cell_start, g.ncells,
                                                                         gs.perm);
-  k_gather_x<TF><<<blocks_for(n, kBlock), kBlock, 0, st>>>(particle_x, gs.perm, n, xs, gs.inv);
+  k_gather_x<TF><<<blocks_for(n, kBlock), kBlock, 0, st>>>(particle_x, gs.perm, n, xs);
   ALB_CUDA(cudaGetLastError());
   return AL_OK;
 }

@@ -21,7 +21,6 @@ struct GridState {
   uint32_t ncells = 0;
   uint32_t* cell = nullptr;        // [n] cell of original particle (kNoCell outside)
   uint32_t* perm = nullptr;        // [n] sorted slot -> original index
-  uint32_t* inv = nullptr;         // [n] original index -> sorted slot
   uint32_t* cell_start = nullptr;  // [ncells + 2]; [ncells] = in-grid count, [ncells+1] = n
   uint32_t* count = nullptr;       // [ncells + 1]; last = out-of-grid count
   uint32_t* flags = nullptr;       // [4] grid_anomaly[0..2] + spare (device)

@@ -9,36 +9,51 @@ namespace {
 
 inline uint32_t blocks_for(uint32_t n, int block) { return (n + block - 1) / block; }
 
+// Threads per particle of the export: eight 16-byte entries (float) fill a
+// 128-byte line of the particle's row.  One thread per particle stored its
+// entries 1 KB apart from its neighbors' lanes: 455 us for 306,525 particles
+// with 64-entry rows, 240 us with eight (B200, whole update).
+constexpr uint32_t kExportLanes = 8;
+
 template <class TF>
 __global__ void k_export_neighbors(Cn<TF> c, uint32_t cap, uint32_t n,
                                    const uint32_t* __restrict__ perm,
-                                   const uint32_t* __restrict__ inv,
                                    const vec4<TF>* __restrict__ xs,
                                    const uint32_t* __restrict__ nbr,
                                    const uint32_t* __restrict__ ncount,
                                    const TF* __restrict__ rho_sorted, TF* __restrict__ out_nbr,
                                    uint32_t* __restrict__ out_num, TF* __restrict__ out_rho) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t s = inv[i];
+  const uint32_t s = blockIdx.x * (blockDim.x / kExportLanes) + threadIdx.x / kExportLanes;
+  const uint32_t lane = threadIdx.x % kExportLanes;
+  if (s >= n) return;
+  const uint32_t i = perm[s];
   const uint32_t cnt = ncount[s];
-  out_num[i] = cnt;
-  if (out_rho) out_rho[i] = rho_sorted[s];
+  if (lane == 0) {
+    out_num[i] = cnt;
+    if (out_rho) out_rho[i] = rho_sorted[s];
+  }
   if (!out_nbr) return;
   const vec3<TF> xi = xyz(xs[s]);
-  for (uint32_t k = 0; k < cnt; ++k) {
-    const uint32_t t = nbr[size_t(k) * n + s];
+  // the caller's buffer may start anywhere
+  const bool aligned = reinterpret_cast<uintptr_t>(out_nbr) % sizeof(vec4<TF>) == 0;
+  for (uint32_t k = lane; k < cnt; k += kExportLanes) {
+    const uint32_t t = nbr[nbr_index(k, s, n)];
     const uint32_t j = perm[t];
     const vec3<TF> xj = xyz(xs[t]);
     TF* e = out_nbr + (size_t(i) * cap + k) * 4;
     const vec3<TF> d = pdisp(c, xi, xj);  // wrapped in y on a periodic update
-    e[0] = d.x;
-    e[1] = d.y;
-    e[2] = d.z;
-    if constexpr (sizeof(TF) == 4) {
-      e[3] = __uint_as_float(j);
+    vec4<TF> w{d.x, d.y, d.z, TF(0)};
+    if constexpr (sizeof(TF) == 4)
+      w.w = __uint_as_float(j);
+    else
+      w.w = __longlong_as_double((long long)j);
+    if (aligned) {
+      *reinterpret_cast<vec4<TF>*>(e) = w;
     } else {
-      e[3] = __longlong_as_double((long long)j);
+      e[0] = w.x;
+      e[1] = w.y;
+      e[2] = w.z;
+      e[3] = w.w;
     }
   }
 }
@@ -79,8 +94,9 @@ int export_neighbors(const Cn<TF>& c, const GridDims& g, const GridState& gs,
                      TF* particle_neighbors, uint32_t* particle_num_neighbors,
                      TF* particle_density, cudaStream_t st) {
   if (gs.n == 0) return AL_OK;
-  k_export_neighbors<TF><<<blocks_for(gs.n, kBlock), kBlock, 0, st>>>(
-      c, g.cap_nbr, gs.n, gs.perm, gs.inv, xs, nbr, ncount, rho_sorted, particle_neighbors,
+  const uint32_t blocks = (gs.n + kBlock / kExportLanes - 1) / (kBlock / kExportLanes);
+  k_export_neighbors<TF><<<blocks, kBlock, 0, st>>>(
+      c, g.cap_nbr, gs.n, gs.perm, xs, nbr, ncount, rho_sorted, particle_neighbors,
       particle_num_neighbors, particle_density);
   ALB_CUDA(cudaGetLastError());
   return AL_OK;

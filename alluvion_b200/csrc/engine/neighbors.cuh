@@ -3,9 +3,10 @@
 // Replaces make_neighbor_list<0> (runner.hpp:1869-1911) and compute_density
 // (runner.hpp:2052-2072).  The reference stores [N][cap] float4 entries
 // {x_i - x_j, j} per particle row; the engine stores 32-bit sorted slots in
-// slot-major layout nbr[k * N + s], so that the k-th neighbor of 32
-// consecutive particles is one coalesced 128-byte line, and recomputes
-// x_i - x_j from the cell-sorted positions (L1/L2 resident) in every pass.
+// groups of kNbrGroup entries, slot-major (nbr_index): one 16-byte load gives
+// a thread four neighbors, 32 consecutive particles read 512 consecutive
+// bytes, and x_i - x_j is recomputed from the cell-sorted positions in every
+// pass.  The last group of a list is padded with the particle's own slot.
 //
 // Candidate order: the 27 cells in ascending linear cell index; the three
 // cells of a (dx, dy) row are contiguous in sorted order, so each row is one
@@ -23,6 +24,16 @@ namespace alb {
 // candidate (the extra bits are masked off), so every sorted-position
 // buffer passed to the build holds n + kSortedPad entries.
 constexpr uint32_t kSortedPad = 8;
+
+// Entries per list group, where entry k of slot s's list lies (row stride
+// `stride` slots), and the words of a list buffer of n slots.
+constexpr uint32_t kNbrGroup = 4;
+__host__ __device__ __forceinline__ size_t nbr_index(uint32_t k, uint32_t s, uint32_t stride) {
+  return (size_t(k / kNbrGroup) * stride + s) * kNbrGroup + k % kNbrGroup;
+}
+inline size_t nbr_list_words(uint32_t n, uint32_t cap) {
+  return size_t(n) * ((size_t(cap) + kNbrGroup - 1) / kNbrGroup * kNbrGroup);
+}
 
 // Boundary kernel terms {grad W * V, W * V} in the reference's
 // [nb][N][4] layout (original particle order); used by the standalone

@@ -29,16 +29,6 @@ template <class TF>
 __device__ __forceinline__ vec4<TF>& RV(const StepState<TF>& S, uint32_t s) {
   return S.rec[2 * size_t(s) + 1];
 }
-// Neighbor loads of the two halves through the read-only path.
-template <class TF>
-__device__ __forceinline__ vec4<TF> gX(const StepState<TF>& S, uint32_t t) {
-  return __ldg(S.rec + 2 * size_t(t));
-}
-template <class TF>
-__device__ __forceinline__ vec4<TF> gV(const StepState<TF>& S, uint32_t t) {
-  return __ldg(S.rec + 2 * size_t(t) + 1);
-}
-
 // Both halves of record t through the read-only path with 256-bit loads
 // (sm_100): one load instruction per float record, two per double record,
 // instead of one per 16 bytes.  Records start on 32-byte (float) and
@@ -175,6 +165,13 @@ __device__ __forceinline__ void scene_bodies(StepState<TF>& S, const BlockSpan& 
   }
 }
 
+// Bodies a block's boundary terms loop over: all `nb` when one of its
+// particles touches a body (mask m), else none, so that the blocks inside the
+// fluid pass one barrier instead of one per body.  All threads call it.
+__device__ __forceinline__ uint32_t block_bodies(uint32_t nb, uint32_t m) {
+  return nb && __syncthreads_or(int(m)) ? nb : 0u;
+}
+
 template <class TF>
 __device__ __forceinline__ Lane pair_lane(const StepState<TF>& S, const BlockSpan& B) {
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -207,62 +204,100 @@ __device__ __forceinline__ vec3<TF> group_sum(vec3<TF> v, const Lane& L) {
   return vec3<TF>{group_sum(v.x, L), group_sum(v.y, L), group_sum(v.z, L)};
 }
 
+// What a pass gathers of each neighbor.  The gathers bound the pair passes:
+// every lane reads its own neighbor, and the L1 data pipe spends about 14
+// cycles on a warp's 16-byte gathers and 28 on its 32-byte ones wherever
+// the neighbors lie (ncu, 1,048,576 particles), so a pass loads no more than
+// it uses: the dense {x, payload} array alone where that is enough.
 template <class TF>
-__device__ __forceinline__ uint32_t nbr_at(const StepState<TF>& S, uint32_t k, uint32_t s) {
-  return __ldcs(S.nbr + size_t(k) * S.ls + s);
+struct NbrXV {
+  vec4<TF> x, v;  // {x, unused}, {v, rho}
+};
+template <class TF>
+struct NbrXS {
+  vec4<TF> x;
+  TF s;
+};
+template <class TF>
+struct LoadX {
+  const vec4<TF>* x;
+  __device__ __forceinline__ vec4<TF> operator()(uint32_t t) const { return __ldg(x + t); }
+};
+template <class TF>
+struct LoadXV {
+  const StepState<TF>& S;
+  __device__ __forceinline__ NbrXV<TF> operator()(uint32_t t) const {
+    NbrXV<TF> r;
+    gXV(S, t, r.x, r.v);
+    return r;
+  }
+};
+
+// Visits the lane's neighbors in list order.  A list is stored in groups of
+// kNbrGroup entries, one 16-byte load each; lane `sub` takes groups sub,
+// sub + tpp, ...  Each round loads the groups of B entries, then gathers
+// `load(t)` of the B entries, then runs `f(t, loaded)` for each.  The
+// entries that pad a list's last group name the particle itself: every pass
+// weighs its neighbors by grad W, which is exactly zero there.  At one thread
+// per particle that is the order of a plain loop over the list; with tpp > 1
+// group_sum combines the lanes' partial sums, a different (fixed) order whose
+// float results differ in the last bits.
+//
+// Against lists with one 4-byte entry per load and bounds tests per entry
+// (35 instead of 56 instructions per neighbor of the kappa passes), with the
+// payload in a dense array instead of the 32-byte records: kappa-style sums
+// 65 instead of 86 us at 1,048,576 particles, 470 instead of 657 us at
+// 8,388,608 (B200, disordered particles, L2 flushed).
+template <int B, class TF, class Load, class F>
+__device__ __forceinline__ void for_each_neighbor(const StepState<TF>& S, const Lane& L,
+                                                  uint32_t cnt, Load&& load, F&& f) {
+  constexpr int kG = B > 4 ? B / 4 : 1;  // groups per round
+  constexpr int kE = B < 4 ? B : 4;      // entries gathered together per group
+  static_assert(kNbrGroup == 4 && (B % 4 == 0 || 4 % B == 0), "rounds of whole groups");
+  const uint4* list = reinterpret_cast<const uint4*>(S.nbr) + L.s;
+  const uint32_t ng = (cnt + kNbrGroup - 1) / kNbrGroup;
+  for (uint32_t g0 = L.sub; g0 < ng; g0 += kG * L.tpp) {
+    uint32_t t[4 * kG];
+#pragma unroll
+    for (int u = 0; u < kG; ++u) {
+      const uint32_t g = g0 + u * L.tpp;
+      uint4 q{L.s, L.s, L.s, L.s};
+      if (u == 0 || g < ng) q = __ldcs(list + size_t(g) * S.ls);
+      t[4 * u] = q.x;
+      t[4 * u + 1] = q.y;
+      t[4 * u + 2] = q.z;
+      t[4 * u + 3] = q.w;
+    }
+#pragma unroll
+    for (int h = 0; h < 4 * kG; h += kE * kG) {
+      decltype(load(0u)) r[kE * kG];
+#pragma unroll
+      for (int b = 0; b < kE * kG; ++b) r[b] = load(t[h + b]);
+#pragma unroll
+      for (int b = 0; b < kE * kG; ++b) f(t[h + b], r[b]);
+    }
+  }
 }
 
-// Visits the lane's neighbors k = sub, sub + tpp, ... < cnt in batches of
-// B: the batch's list entries are loaded first, then all their records,
-// then `f(t, x_j, v_j)` runs for each in list order.  At one thread per
-// particle that is the order of a plain loop over the list, so sums are
-// bit-identical to one; with tpp > 1 each lane sums every tpp-th neighbor
-// and group_sum combines the partial sums, a different (fixed) order whose
-// float results differ in the last bits.  Batching keeps B dependent
-// index -> record chains in flight per lane; it pays in the passes with
-// much arithmetic per neighbor (measured on the 1M-particle dam break at
-// one thread per particle: B = 8 for k_kappa (1.922 vs 1.928 ms per step at
-// 4, 1.946 at 2), 4 for viscosity, 2 for the velocity-divergence passes,
-// which have little arithmetic per neighbor).  `v_j` is loaded only when
-// V.
-template <int B, bool V, class TF, class F>
-__device__ __forceinline__ void for_each_neighbor(const StepState<TF>& S, const Lane& L,
-                                                  uint32_t cnt, F&& f) {
-  for (uint32_t k0 = L.sub; k0 < cnt; k0 += B * L.tpp) {
-    uint32_t t[B];
-#pragma unroll
-    for (int b = 0; b < B; ++b) {
-      const uint32_t k = k0 + b * L.tpp;
-      t[b] = k < cnt ? nbr_at(S, k, L.s) : L.s;  // own slot: a valid address
-    }
-    vec4<TF> xj[B], vj[B];
-#pragma unroll
-    for (int b = 0; b < B; ++b) {
-      if (V) {
-        gXV(S, t[b], xj[b], vj[b]);
-      } else {
-        xj[b] = gX(S, t[b]);
-        vj[b] = vec4<TF>{0, 0, 0, 0};
-      }
-    }
-#pragma unroll
-    for (int b = 0; b < B; ++b)
-      if (k0 + b * L.tpp < cnt) f(t[b], xj[b], vj[b]);
-  }
+// Records a velocity-divergence pass gathers together: four float ones, two
+// with the periodic wrap or in double, whose records are 64 bytes.
+template <class TF, bool WR>
+constexpr int xv_batch() {
+  return sizeof(TF) == 4 && !WR ? 4 : 2;
 }
 
 // Sum over neighbors of V (v_i - v_j) . grad W_ij plus the boundary terms
 // (v_i - v_b) . (grad W V)_b: the shared body of compute_density_change
 // (runner.hpp:3192-3228) and compute_density_adv (runner.hpp:3493-3523).
 // Every lane of the group calls it and receives the full sum.
-template <class TF>
+template <bool WR, class TF>
 __device__ __forceinline__ TF velocity_divergence(const Cn<TF>& c, const StepState<TF>& S,
                                                   const Lane& L, vec3<TF> xi, vec3<TF> vi,
                                                   uint32_t cnt) {
   TF acc = 0;
-  for_each_neighbor<2, true>(S, L, cnt, [&](uint32_t, const vec4<TF>& xj, const vec4<TF>& vj) {
-    const vec3<TF> d = pdisp(c, xi, xyz(xj));
-    acc += c.vol * dot(vi - xyz(vj), gradW(c, d));
+  for_each_neighbor<xv_batch<TF, WR>()>(S, L, cnt, LoadXV<TF>{S}, [&](uint32_t, const NbrXV<TF>& r) {
+    const vec3<TF> d = pdisp(c, xi, xyz(r.x));
+    acc += c.vol * dot(vi - xyz(r.v), gradW(c, d));
   });
   acc = group_sum(acc, L);
   if (L.act) {
@@ -277,25 +312,25 @@ __device__ __forceinline__ TF velocity_divergence(const Cn<TF>& c, const StepSta
   return acc;
 }
 
-template <class TF>
+template <bool WR, class TF>
 __device__ __forceinline__ TF density_change(const Cn<TF>& c, const StepState<TF>& S,
                                              const Lane& L) {
   const uint32_t cnt = L.act ? S.ncount[L.s] : 0u;
   const vec3<TF> xi = L.act ? xyz(RX(S, L.s)) : vec3<TF>{0, 0, 0};
   const vec3<TF> vi = L.act ? xyz(RV(S, L.s)) : vec3<TF>{0, 0, 0};
-  TF adv = velocity_divergence(c, S, L, xi, vi, cnt);
+  TF adv = velocity_divergence<WR>(c, S, L, xi, vi, cnt);
   adv = fmax(adv, TF(0));
   if (cnt < 20) adv = 0;
   return adv;
 }
 
-template <class TF>
+template <bool WR, class TF>
 __device__ __forceinline__ TF density_adv(const Cn<TF>& c, const StepState<TF>& S, const Lane& L,
                                           TF dt) {
   const uint32_t cnt = L.act ? S.ncount[L.s] : 0u;
   const vec3<TF> xi = L.act ? xyz(RX(S, L.s)) : vec3<TF>{0, 0, 0};
   const vec3<TF> vi = L.act ? xyz(RV(S, L.s)) : vec3<TF>{0, 0, 0};
-  const TF delta = velocity_divergence(c, S, L, xi, vi, cnt);
+  const TF delta = velocity_divergence<WR>(c, S, L, xi, vi, cnt);
   const TF rho = L.act ? S.rho[L.s] : c.rho0;
   return fmax(rho / c.rho0 + dt * delta, TF(1));
 }
@@ -378,7 +413,7 @@ struct WarmDivergence {
     const TF kv = S.kappa_v[s];
     const TF w = adv > TF(0) ? TF(0.5) * fmax(kv, TF(-0.5)) / dt : TF(0);
     S.kappa_v[s] = w;
-    RX(S, s).w = w;
+    S.x[s].w = w;
     const bool learned = feat && !(floor && *floor);
     if (learned || feat_out) {
       const TF speed = sqrt(length_sqr(o.vi));
@@ -439,7 +474,7 @@ __global__ void k_apply_warm_div(StepState<TF> S, const float* __restrict__ feat
   if (s >= S.n || *floor) return;
   const TF w = feat[size_t(s) * AL_WARM_NUM_FEATURES + 1] > 0.f ? TF(pred[2 * size_t(s)]) : TF(0);
   S.kappa_v[s] = w;
-  RX(S, s).w = w;
+  S.x[s].w = w;
 }
 
 enum KappaMode { kDivWarm = 0, kDivIter = 1, kPressWarm = 2, kPressIter = 3 };
@@ -448,11 +483,8 @@ enum KappaMode { kDivWarm = 0, kDivIter = 1, kPressWarm = 2, kPressIter = 3 };
 // (runner.hpp:3251-3295), divergence_solve_iteration (:3316-3363),
 // warm_start_pressure_solve1 (:3451-3491), pressure_solve_iteration
 // (:3543-3588).  Boundary reaction forces go to the per-block rigid slots.
-// The float kernel is held at 56 registers (9 resident 128-thread blocks
-// per SM; with 256-thread launch bounds the compiler took 58, and the
-// 256-register allocation granule then allows only 8); double needs more.
 template <class TF, int MODE, bool WR = false, bool BT = false>
-__global__ void __maxnreg__(sizeof(TF) == 4 ? 56 : 128) k_kappa(Cn<TF> c, StepState<TF> S) {
+__global__ void __launch_bounds__(kMaxBlock) k_kappa(Cn<TF> c, StepState<TF> S) {
   if constexpr (!WR) c.wrap = 0;  // non-periodic: the wrap branches fold away
   constexpr bool kDiv = MODE == kDivWarm || MODE == kDivIter;
   BlockSpan B;
@@ -467,12 +499,12 @@ __global__ void __maxnreg__(sizeof(TF) == 4 ? 56 : 128) k_kappa(Cn<TF> c, StepSt
   uint32_t cnt = 0;
   vec3<TF> xi{0, 0, 0};
   if (L.act) {
-    const vec4<TF> r = RX(S, L.s);
+    const vec4<TF> r = S.x[L.s];
     ki = r.w;
     xi = xyz(r);
     cnt = S.ncount[L.s];
   }
-  for_each_neighbor<8, false>(S, L, cnt, [&](uint32_t, const vec4<TF>& xj, const vec4<TF>&) {
+  for_each_neighbor<4>(S, L, cnt, LoadX<TF>{S.x}, [&](uint32_t, const vec4<TF>& xj) {
     const TF ksum = ki + xj.w;
     if (fabs(ksum) > c.eps) {
       const vec3<TF> gw = gradW(c, pdisp(c, xi, xyz(xj)));
@@ -487,7 +519,8 @@ __global__ void __maxnreg__(sizeof(TF) == 4 ? 56 : 128) k_kappa(Cn<TF> c, StepSt
   dv = group_sum(dv, L);
   scene_bodies<BT>(S, B);
   const uint32_t m = (L.lead() && fabs(ki) > c.eps) ? S.mask[L.s] : 0u;
-  for (uint32_t b = 0; b < S.nb; ++b) {
+  const uint32_t nb = block_bodies(S.nb, m);
+  for (uint32_t b = 0; b < nb; ++b) {
     const bool mine = (m >> b) & 1u;
     if (!__syncthreads_or(mine)) continue;
     vec3<TF> f{0, 0, 0}, tq{0, 0, 0};
@@ -518,13 +551,13 @@ __global__ void __launch_bounds__(kMaxBlock) k_df_rho_adv_init(Cn<TF> c, StepSta
   if (!block_scene<BT>(S, B)) return;
   scene_bodies<BT>(S, B);
   const Lane L = pair_lane(S, B);
-  const TF adv = density_change(c, S, L);
+  const TF adv = density_change<WR>(c, S, L);
   if (!L.lead()) return;
   const TF dt = S.ctrl->dt;
   const TF alpha = S.alpha[L.s] * (TF(1) / dt);
   S.rho_adv[L.s] = adv;
   S.alpha[L.s] = alpha;
-  RX(S, L.s).w = adv * alpha;
+  S.x[L.s].w = adv * alpha;
 }
 
 // compute_divergence_solve_density_error (runner.hpp:3396-3410) with the
@@ -538,11 +571,11 @@ __global__ void __launch_bounds__(kMaxBlock)
   if (BT && !S.ctrl->keep_going) return;
   scene_bodies<BT>(S, B);
   const Lane L = pair_lane(S, B);
-  const TF adv = density_change(c, S, L);
+  const TF adv = density_change<WR>(c, S, L);
   double val = 0;
   if (L.lead()) {
     S.rho_adv[L.s] = adv;
-    RX(S, L.s).w = adv * S.alpha[L.s];
+    S.x[L.s].w = adv * S.alpha[L.s];
     val = double(adv);
   }
   double total;
@@ -572,16 +605,18 @@ __global__ void __launch_bounds__(kMaxBlock, sizeof(TF) == 4 ? 4 : 1)
     vi = xyz(RV(S, L.s));
     cnt = S.ncount[L.s];
   }
-  for_each_neighbor<4, true>(S, L, cnt, [&](uint32_t, const vec4<TF>& xj, const vec4<TF>& vj) {
-    const vec3<TF> d = pdisp(c, xi, xyz(xj));  // vj = {v, rho}
-    da += (c.visc * c.mass / vj.w * dot(d, gradW(c, d)) /
-           (length_sqr(d) + TF(0.01) * c.h2)) *
-          (vi - xyz(vj));
+  for_each_neighbor<xv_batch<TF, WR>()>(S, L, cnt, LoadXV<TF>{S},
+                                        [&](uint32_t, const NbrXV<TF>& r) {
+    const vec3<TF> d = pdisp(c, xi, xyz(r.x));  // r.v = {v, rho}
+    da += (c.visc * c.mass * dot(d, gradW(c, d)) /
+           (r.v.w * (length_sqr(d) + TF(0.01) * c.h2))) *
+          (vi - xyz(r.v));
   });
   da = group_sum(da, L);
   scene_bodies<BT>(S, B);
   const uint32_t m = L.lead() ? S.mask[L.s] : 0u;
-  for (uint32_t b = 0; b < S.nb; ++b) {
+  const uint32_t nb = block_bodies(S.nb, m);
+  for (uint32_t b = 0; b < nb; ++b) {
     const bool mine = (m >> b) & 1u;
     if (!__syncthreads_or(mine)) continue;
     vec3<TF> fsum{0, 0, 0}, tsum{0, 0, 0};
@@ -694,7 +729,7 @@ __global__ void __launch_bounds__(kMaxBlock)
   scene_bodies<BT>(S, B);
   const Lane L = pair_lane(S, B);
   const TF dt = S.ctrl->dt;
-  const TF adv = density_adv(c, S, L, dt);
+  const TF adv = density_adv<WR>(c, S, L, dt);
   if (!L.lead()) return;
   const TF kp = S.kappa[L.s];
   const bool learned = pred && !(floor && *floor);
@@ -702,7 +737,7 @@ __global__ void __launch_bounds__(kMaxBlock)
                        : TF(0.5) * fmax(kp, TF(-0.00025)) / (dt * dt);
   const TF w = adv > TF(1) ? warm : TF(0);
   S.kappa[L.s] = w;
-  RX(S, L.s).w = w;
+  S.x[L.s].w = w;
 }
 
 // compute_rho_adv (runner.hpp:3525-3541); also k for the first iteration.
@@ -714,12 +749,12 @@ __global__ void __launch_bounds__(kMaxBlock) k_p_rho_adv_init(Cn<TF> c, StepStat
   scene_bodies<BT>(S, B);
   const Lane L = pair_lane(S, B);
   const TF dt = S.ctrl->dt;
-  const TF adv = density_adv(c, S, L, dt);
+  const TF adv = density_adv<WR>(c, S, L, dt);
   if (!L.lead()) return;
   const TF alpha = S.alpha[L.s] * (TF(1) / (dt * dt));
   S.rho_adv[L.s] = adv;
   S.alpha[L.s] = alpha;
-  RX(S, L.s).w = (adv - TF(1)) * alpha;
+  S.x[L.s].w = (adv - TF(1)) * alpha;
 }
 
 // compute_pressure_solve_density_error (runner.hpp:3590-3604); the mean is
@@ -733,11 +768,11 @@ __global__ void __launch_bounds__(kMaxBlock)
   if (BT && !S.ctrl->keep_going) return;
   scene_bodies<BT>(S, B);
   const Lane L = pair_lane(S, B);
-  const TF adv = density_adv(c, S, L, S.ctrl->dt);
+  const TF adv = density_adv<WR>(c, S, L, S.ctrl->dt);
   double val = 0;
   if (L.lead()) {
     S.rho_adv[L.s] = adv;
-    RX(S, L.s).w = (adv - TF(1)) * S.alpha[L.s];
+    S.x[L.s].w = (adv - TF(1)) * S.alpha[L.s];
     val = double(adv) - 1.0;
   }
   double total;
@@ -809,8 +844,9 @@ __global__ void __launch_bounds__(kMaxBlock) k_ii_predict0(Cn<TF> c, StepState<T
     cnt = S.ncount[L.s];
   }
   vec3<TF> dii{0, 0, 0};
-  for_each_neighbor<4, false>(S, L, cnt, [&](uint32_t, const vec4<TF>& xj, const vec4<TF>&) {
-    dii -= (c.vol / rho2) * gradW(c, pdisp(c, xi, xyz(xj)));
+  const TF vr = c.vol / rho2;
+  for_each_neighbor<4>(S, L, cnt, LoadX<TF>{S.x}, [&](uint32_t, const vec4<TF>& xj) {
+    dii -= vr * gradW(c, pdisp(c, xi, xyz(xj)));
   });
   dii = group_sum(dii, L);
   if (!L.lead()) return;
@@ -820,7 +856,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_ii_predict0(Cn<TF> c, StepState<T
   RV(S, L.s) = vec4<TF>{v.x + dt * a.x, v.y + dt * a.y, v.z + dt * a.z, v.w};
   const TF lp = S.kappa[L.s] * TF(0.5);
   S.kappa_v[L.s] = lp;
-  RX(S, L.s).w = lp;  // pressure read by the first iteration
+  S.x[L.s].w = lp / rho2;  // read by the first iteration
   for (uint32_t m = S.mask[L.s]; m; m &= m - 1) {
     const uint32_t b = __ffs(m) - 1;
     const vec4<TF> kg = S.bk[size_t(b) * S.ls + L.s];
@@ -848,10 +884,11 @@ __global__ void __launch_bounds__(kMaxBlock) k_ii_predict1(Cn<TF> c, StepState<T
   }
   const TF rho2 = rho * rho, inv_rho2 = TF(1) / rho2, dpi = c.vol * inv_rho2;
   TF adv = 0, aii = 0;
-  for_each_neighbor<4, true>(S, L, cnt, [&](uint32_t, const vec4<TF>& xj, const vec4<TF>& vj) {
-    const vec3<TF> gw = gradW(c, pdisp(c, xi, xyz(xj)));
+  for_each_neighbor<xv_batch<TF, WR>()>(S, L, cnt, LoadXV<TF>{S},
+                                        [&](uint32_t, const NbrXV<TF>& r) {
+    const vec3<TF> gw = gradW(c, pdisp(c, xi, xyz(r.x)));
     const vec3<TF> dji = (dpi * c.rho0) * gw;
-    adv += dt * c.vol * dot(vi - xyz(vj), gw);
+    adv += dt * c.vol * dot(vi - xyz(r.v), gw);
     aii += c.vol * dot(dii - dji, gw);
   });
   adv = group_sum(adv, L);
@@ -874,7 +911,9 @@ __global__ void __launch_bounds__(kMaxBlock) k_ii_predict1(Cn<TF> c, StepState<T
 // pressure_solve_iteration0 (runner.hpp:2691-2715).  On iterations after
 // the first, also performs the reference's last_pressure <- pressure copy
 // (solver_ii.hpp:204) for the own particle; this kernel reads the
-// neighbors' pressure (equal to their last pressure after that copy).
+// neighbors' pressure (equal to their last pressure after that copy) as the
+// payload p / rho^2.  Besides sum_j d_ij p_j it writes what the neighbors
+// need of it next, sum_j d_ij p_j + d_ii p_i, as one vector.
 template <class TF, bool WR = false>
 __global__ void __launch_bounds__(kMaxBlock) k_ii_iter0(Cn<TF> c, StepState<TF> S) {
   if constexpr (!WR) c.wrap = 0;  // non-periodic: the wrap branches fold away
@@ -887,17 +926,19 @@ __global__ void __launch_bounds__(kMaxBlock) k_ii_iter0(Cn<TF> c, StepState<TF> 
     cnt = S.ncount[L.s];
   }
   // the payload holds the last pressure on the first iteration
-  // (k_ii_predict0) and the pressure afterwards (k_ii_iter1)
+  // (k_ii_predict0) and the pressure afterwards (k_ii_iter1), over rho^2
   vec3<TF> acc{0, 0, 0};
-  for_each_neighbor<4, true>(S, L, cnt, [&](uint32_t, const vec4<TF>& xj, const vec4<TF>& vj) {
-    const TF rj = vj.w, rj2 = rj * rj;
-    acc -= (c.vol / rj2 * xj.w) * gradW(c, pdisp(c, xi, xyz(xj)));
+  for_each_neighbor<4>(S, L, cnt, LoadX<TF>{S.x}, [&](uint32_t, const vec4<TF>& xj) {
+    acc -= (c.vol * xj.w) * gradW(c, pdisp(c, xi, xyz(xj)));
   });
   acc = group_sum(acc, L);
   if (!L.lead()) return;
-  if (!first) S.kappa_v[L.s] = S.kappa[L.s];
+  const TF lp = first ? S.kappa_v[L.s] : S.kappa[L.s];
+  if (!first) S.kappa_v[L.s] = lp;
   acc = acc * c.rho0;
   S.dij_pj[L.s] = vec4<TF>{acc.x, acc.y, acc.z, TF(0)};
+  const vec3<TF> q = acc + lp * xyz(S.dii[L.s]);
+  S.dq[L.s] = vec4<TF>{q.x, q.y, q.z, TF(0)};
 }
 
 // pressure_solve_iteration1 (runner.hpp:2716-2772) and the mean of
@@ -920,12 +961,13 @@ __global__ void __launch_bounds__(kMaxBlock)
   }
   const TF rho2 = rho * rho, dpi = c.vol / rho2;
   TF sum = 0;
-  for_each_neighbor<4, false>(S, L, cnt, [&](uint32_t t, const vec4<TF>& xj, const vec4<TF>&) {
-    const vec3<TF> gw = gradW(c, pdisp(c, xi, xyz(xj)));
-    const vec3<TF> dji = (dpi * c.rho0) * gw;
-    const vec3<TF> dji_pi = dji * lp;
-    sum += c.vol *
-           dot(dij_pj - ldx(S.dii, t) * __ldg(S.kappa_v + t) - (ldx(S.dij_pj, t) - dji_pi), gw);
+  const TF dpi_pi = dpi * c.rho0 * lp;  // d_ji p_i = dpi_pi grad W
+  auto load = [&](uint32_t t) {
+    return NbrXV<TF>{__ldg(S.x + t), __ldg(S.dq + t)};  // {x, payload}, {d_jj p_j + sum_k d_jk p_k}
+  };
+  for_each_neighbor<4>(S, L, cnt, load, [&](uint32_t, const NbrXV<TF>& r) {
+    const vec3<TF> gw = gradW(c, pdisp(c, xi, xyz(r.x)));
+    sum += c.vol * dot(dij_pj - xyz(r.v) + dpi_pi * gw, gw);
   });
   sum = group_sum(sum, L);
   double val = 0;
@@ -943,9 +985,8 @@ __global__ void __launch_bounds__(kMaxBlock)
     if (fabs(denom) > TF(1.0e-9))
       p = fmax((TF(1) - omega) * lp + omega / denom * (bterm - dt2 * sum), TF(0));
     const TF err = p == TF(0) ? TF(0) : (denom * p + sum * dt2 - bterm);
-    S.err[L.s] = err;
     S.kappa[L.s] = p;
-    RX(S, L.s).w = p;  // pressure read by the next iteration
+    S.x[L.s].w = p / rho2;  // read by the next iteration and the accelerations
     val = double(err);
   }
   double total;
@@ -962,6 +1003,9 @@ __global__ void __launch_bounds__(kMaxBlock)
                       TF* __restrict__ rho_adv_ref) {
   if constexpr (!WR) c.wrap = 0;  // non-periodic: the wrap branches fold away
   const Lane L = pair_lane(S);
+  // a solve of no iterations leaves the caller's pressure, which is not the
+  // payload's
+  const bool none = S.ctrl->it == 0;
   vec3<TF> ai{0, 0, 0}, xi{0, 0, 0};
   TF dpi = 0;
   uint32_t cnt = 0;
@@ -971,14 +1015,18 @@ __global__ void __launch_bounds__(kMaxBlock)
     dpi = S.kappa[L.s] / (rho * rho);
     cnt = S.ncount[L.s];
   }
-  for_each_neighbor<4, true>(S, L, cnt, [&](uint32_t t, const vec4<TF>& xj, const vec4<TF>& vj) {
-    const TF rj = vj.w;
-    const TF dpj = __ldg(S.kappa + t) / (rj * rj);
+  for_each_neighbor<4>(S, L, cnt, LoadX<TF>{S.x}, [&](uint32_t t, const vec4<TF>& xj) {
+    TF dpj = xj.w;  // p / rho^2
+    if (none) {
+      const TF rj = __ldg(S.rho + t);
+      dpj = __ldg(S.kappa + t) / (rj * rj);
+    }
     ai -= (c.mass * (dpi + dpj)) * gradW(c, pdisp(c, xi, xyz(xj)));
   });
   ai = group_sum(ai, L);
   const uint32_t m = L.lead() ? S.mask[L.s] : 0u;
-  for (uint32_t b = 0; b < S.nb; ++b) {
+  const uint32_t nb = block_bodies(S.nb, m);
+  for (uint32_t b = 0; b < nb; ++b) {
     const bool mine = (m >> b) & 1u;
     if (!__syncthreads_or(mine)) continue;
     vec3<TF> f{0, 0, 0}, tq{0, 0, 0};
@@ -1008,7 +1056,7 @@ __global__ void __launch_bounds__(kMaxBlock)
 
 // ---------------------------------------------------- implicit SPH (SolverI)
 // advect_and_init_pressure (runner.hpp:2889-2900): v += dt a, last pressure
-// (kappa_v) = pressure / 2.
+// (kappa_v) = pressure / 2; also the iterations' payload arrays and 1 / rho.
 template <class TF>
 __global__ void __launch_bounds__(kMaxBlock) k_i_advect(StepState<TF> S) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1017,7 +1065,12 @@ __global__ void __launch_bounds__(kMaxBlock) k_i_advect(StepState<TF> S) {
   const vec4<TF> a = S.a[s];
   const vec4<TF> v = RV(S, s);
   RV(S, s) = vec4<TF>{v.x + dt * a.x, v.y + dt * a.y, v.z + dt * a.z, v.w};
-  S.kappa_v[s] = S.kappa[s] * TF(0.5);
+  const TF lp = S.kappa[s] * TF(0.5);
+  S.kappa_v[s] = lp;
+  const vec4<TF> x = S.x[s];
+  S.x[s].w = lp;
+  S.x1[s] = vec4<TF>{x.x, x.y, x.z, TF(0)};
+  S.irho[s] = TF(1) / S.rho[s];
 }
 
 // calculate_isph_diagonal_adv_density (runner.hpp:2901-2954): the Jacobi
@@ -1038,12 +1091,13 @@ __global__ void __launch_bounds__(kMaxBlock) k_i_diag(Cn<TF> c, StepState<TF> S)
   }
   const TF eps = TF(0.01) * c.h2;
   TF adv = 0, diag = 0;
-  for_each_neighbor<4, true>(S, L, cnt, [&](uint32_t, const vec4<TF>& xj, const vec4<TF>& vj) {
-    const vec3<TF> d = pdisp(c, xi, xyz(xj));  // vj = {v, rho}
+  for_each_neighbor<xv_batch<TF, WR>()>(S, L, cnt, LoadXV<TF>{S},
+                                        [&](uint32_t, const NbrXV<TF>& r) {
+    const vec3<TF> d = pdisp(c, xi, xyz(r.x));  // r.v = {v, rho}
     const vec3<TF> gw = gradW(c, d);
-    const TF rj = vj.w;
-    adv += dt * c.vol * dot(vi - xyz(vj), gw);
-    diag += c.vol * (rho + rj) / (rho * rj) / (length_sqr(d) + eps) * dot(d, gw);
+    const TF rj = r.v.w;
+    adv += dt * c.vol * dot(vi - xyz(r.v), gw);
+    diag += c.vol * (rho + rj) * dot(d, gw) / (rho * rj * (length_sqr(d) + eps));
   });
   adv = group_sum(adv, L);
   diag = group_sum(diag, L);
@@ -1066,7 +1120,9 @@ __global__ void __launch_bounds__(kMaxBlock) k_i_diag(Cn<TF> c, StepState<TF> S)
 // solver_i.hpp:272-274 (double, on the device).  The reference copies
 // pressure into last_pressure after each iteration; here the two arrays
 // swap roles by iteration parity: iteration k reads kappa_v and writes
-// kappa when k is even, the reverse when odd.
+// kappa when k is even, the reverse when odd, and so do the arrays x and x1
+// whose payload holds the pressure the neighbors read (16 + 4 bytes gathered
+// per neighbor, with 1 / rho, instead of the record's 32 and the pressure's 4).
 template <class TF, bool WR = false>
 __global__ void __launch_bounds__(kMaxBlock)
     k_i_iter(Cn<TF> c, StepState<TF> S, cudaGraphConditionalHandle handle, int use_handle) {
@@ -1076,22 +1132,23 @@ __global__ void __launch_bounds__(kMaxBlock)
   const bool odd = (S.ctrl->it & 1u) != 0;
   const TF* __restrict__ last = odd ? S.kappa : S.kappa_v;
   TF* __restrict__ next = odd ? S.kappa_v : S.kappa;
+  const vec4<TF>* xl = odd ? S.x1 : S.x;
+  vec4<TF>* xn = odd ? S.x : S.x1;
   vec3<TF> xi{0, 0, 0};
-  TF rho = c.rho0, lp = 0;
+  TF irho = 0, lp = 0;
   uint32_t cnt = 0;
   if (L.act) {
     xi = xyz(RX(S, L.s));
-    rho = S.rho[L.s];
+    irho = S.irho[L.s];
     lp = last[L.s];
     cnt = S.ncount[L.s];
   }
   const TF eps = TF(0.01) * c.h2;
   TF off = 0;
-  for_each_neighbor<4, true>(S, L, cnt, [&](uint32_t t, const vec4<TF>& xj, const vec4<TF>& vj) {
-    const vec3<TF> d = pdisp(c, xi, xyz(xj));
-    const TF rj = vj.w;
-    off -= c.vol * (rho + rj) / (rho * rj) / (length_sqr(d) + eps) * dot(d, gradW(c, d)) *
-           __ldg(last + t);
+  auto load = [&](uint32_t t) { return NbrXS<TF>{__ldg(xl + t), __ldg(S.irho + t)}; };
+  for_each_neighbor<4>(S, L, cnt, load, [&](uint32_t, const NbrXS<TF>& r) {
+    const vec3<TF> d = pdisp(c, xi, xyz(r.x));  // (rho_i + rho_j) / (rho_i rho_j) = 1/rho_i + 1/rho_j
+    off -= c.vol * (irho + r.s) * dot(d, gradW(c, d)) / (length_sqr(d) + eps) * r.x.w;
   });
   off = group_sum(off, L);
   double val = 0;
@@ -1106,8 +1163,8 @@ __global__ void __launch_bounds__(kMaxBlock)
     if (fabs(denom) > TF(1.0e-9))
       p = fmax((TF(1) - w) * lp + w * (bterm / denom - off / diag), TF(0));
     const TF err = p == TF(0) ? TF(0) : (denom * p + off * dt2 - bterm);
-    S.err[L.s] = err;
     next[L.s] = p;
+    xn[L.s].w = p;
     val = double(err);
   }
   double total;
@@ -1116,13 +1173,18 @@ __global__ void __launch_bounds__(kMaxBlock)
 }
 
 // After an even, non-zero number of iterations the final pressure sits in
-// kappa_v: move it to kappa, where the acceleration pass reads it.
+// kappa_v: move it to kappa, where the acceleration pass reads it, and make
+// p / rho^2 the payload that pass gathers.
 template <class TF>
 __global__ void k_i_final(StepState<TF> S) {
   const uint32_t it = S.ctrl->it;
-  if (it == 0 || (it & 1u)) return;
-  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < S.n; s += gridDim.x * blockDim.x)
-    S.kappa[s] = S.kappa_v[s];
+  if (it == 0) return;
+  for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < S.n; s += gridDim.x * blockDim.x) {
+    const TF p = (it & 1u) ? S.kappa[s] : S.kappa_v[s];
+    if (!(it & 1u)) S.kappa[s] = p;
+    const TF rho = S.rho[s];
+    S.x[s].w = p / (rho * rho);
+  }
 }
 
 // ------------------------------------------------------------ host side
@@ -1759,13 +1821,17 @@ int prepare_step(al_engine* e, const StepArgs<TF>& A, StepPlan<TF>& P, uint32_t 
     ALB_TRY(e->buf("sorted.kappa_v", n, &S.kappa_v));
     if (iisph) {
       ALB_TRY(e->buf("sorted.kk", n, &S.kk));
-      ALB_TRY(e->buf("sorted.err", n, &S.err));
     }
     if (iisph && !P.isph) {
       ALB_TRY(e->buf("sorted.dii", n, &S.dii));
       ALB_TRY(e->buf("sorted.dij_pj", n, &S.dij_pj));
+      ALB_TRY(e->buf("sorted.dq", n, &S.dq));
     }
-    ALB_TRY(e->buf("nbr.list", size_t(n) * P.g.cap_nbr, &S.nbr));
+    if (P.isph) {
+      ALB_TRY(e->buf("sorted.x1", n, &S.x1));
+      ALB_TRY(e->buf("sorted.irho", n, &S.irho));
+    }
+    ALB_TRY(e->buf("nbr.list", nbr_list_words(n, P.g.cap_nbr), &S.nbr));
     ALB_TRY(e->buf("nbr.count", n, &S.ncount));
     ALB_TRY(e->buf("bnd.mask", n, &S.mask));
     ALB_TRY(e->buf("bnd.x", size_t(nb ? nb : 1) * n, &S.bx));
@@ -2178,7 +2244,7 @@ int fused_prepare(al_engine* e, std::vector<StepPlan<TF>>& plans, FusedPlan<TF>&
   ALB_TRY(e->buf("sorted.rho_adv", N, &A.rho_adv));
   ALB_TRY(e->buf("sorted.kappa", N, &A.kappa));
   ALB_TRY(e->buf("sorted.kappa_v", N, &A.kappa_v));
-  ALB_TRY(e->buf("nbr.list", size_t(N) * cap, &A.nbr));
+  ALB_TRY(e->buf("nbr.list", nbr_list_words(uint32_t(N), cap), &A.nbr));
   ALB_TRY(e->buf("nbr.count", N, &A.ncount));
   ALB_TRY(e->buf("bnd.mask", N, &A.mask));
   ALB_TRY(e->buf("bnd.x", size_t(nbmax) * N, &A.bx));
@@ -2226,7 +2292,7 @@ int fused_prepare(al_engine* e, std::vector<StepPlan<TF>>& plans, FusedPlan<TF>&
     Sk.rho_adv = A.rho_adv + o;
     Sk.kappa = A.kappa + o;
     Sk.kappa_v = A.kappa_v + o;
-    Sk.nbr = A.nbr + o;
+    Sk.nbr = A.nbr + kNbrGroup * size_t(o);
     Sk.ncount = A.ncount + o;
     Sk.mask = A.mask + o;
     Sk.bx = A.bx + o;

@@ -55,18 +55,20 @@ template <class TF>
 struct StepState {
   uint32_t n = 0, nb = 0, cap = 0, grid = 0;
   uint32_t tpp = 1;  // threads per particle of the pair passes (pair_tpp)
-  // Stride of the slot-major arrays (nbr [cap][ls], bx / bk [nb][ls]): n for
+  // Stride of the slot-major arrays (nbr [cap / 4][ls][4], bx / bk [nb][ls]): n for
   // one scene; the arena's particle count for the scenes of a fused batch.
   uint32_t ls = 0;
-  vec4<TF>* x = nullptr;    // sorted positions (grid sort, boundaries, build)
-  // Interleaved particle records of the pair passes: rec[2s] = {x, payload},
-  // rec[2s + 1] = {v, rho}.  One 32-byte sector (float) holds all a
-  // neighbor contributes to any DFSPH pass.  `payload` is the scalar the
-  // next k_kappa pass reads from its neighbors (the kappa_v / kappa warm
-  // start, or k = b alpha of the running iteration); the kernels that write
-  // it read only x from the same half, so the 4-byte store never races
-  // with a value another thread uses.
+  // Sorted positions with a payload {x, payload}: what the passes gather
+  // that need one scalar of each neighbor.  `payload` is the scalar the next
+  // such pass reads (the kappa_v / kappa warm start, or k = b alpha of the
+  // running iteration; p / rho^2 in IISPH, the last pressure in implicit
+  // SPH); the kernels that write it read only x from its neighbors, so the
+  // 4-byte store never races with a value another thread uses.
+  vec4<TF>* x = nullptr;
+  // Interleaved particle records of the passes that gather velocities:
+  // rec[2s] = {x, unused}, rec[2s + 1] = {v, rho}, one 32-byte sector (float).
   vec4<TF>* rec = nullptr;
+  vec4<TF>* x1 = nullptr;  // implicit SPH: x with the payload of odd iterations
   vec4<TF>* a = nullptr;
   TF* rho = nullptr;
   TF* alpha = nullptr;
@@ -74,9 +76,10 @@ struct StepState {
   TF* kappa = nullptr;    // DFSPH kappa, IISPH / implicit SPH pressure
   TF* kappa_v = nullptr;  // DFSPH kappa_v, IISPH / implicit SPH last pressure
   TF* kk = nullptr;       // IISPH aii, implicit SPH diagonal (times rho0)
-  TF* err = nullptr;      // IISPH / implicit SPH density error
+  TF* irho = nullptr;     // implicit SPH 1 / rho
   vec4<TF>* dii = nullptr;
   vec4<TF>* dij_pj = nullptr;
+  vec4<TF>* dq = nullptr;   // IISPH sum_k d_jk p_k + d_jj p_j
   uint32_t* nbr = nullptr;
   uint32_t* ncount = nullptr;
   uint32_t* mask = nullptr;
