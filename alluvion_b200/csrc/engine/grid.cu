@@ -1,4 +1,4 @@
-// grid.cu -- cell hash, 3-pass exclusive scan, stable counting sort.
+// grid.cu -- cell hash, exclusive scan, stable counting sort.
 #include "grid.cuh"
 
 namespace alb {
@@ -126,6 +126,49 @@ __global__ void k_scan_add(uint32_t* __restrict__ start, uint32_t len,
   if (idx < len) start[idx] += sums[idx / kScanTile];
 }
 
+// Phases 2 and 3 in one launch, one block per tile: the block sums the
+// totals of the tiles before its own and adds them to its entries.  Its reads
+// grow with the square of the tile count, so it serves up to kFinishTiles
+// tiles (8.4 M cells; 4,096 totals are 16 KB per block), where it saves a
+// launch, which is what a scan of few tiles costs (about 4 us in a step graph).
+constexpr uint32_t kFinishTiles = 4096;
+
+__global__ void __launch_bounds__(kScanThreads)
+    k_scan_finish(uint32_t* __restrict__ start, uint32_t len, const uint32_t* __restrict__ sums) {
+  __shared__ uint32_t part[kScanThreads / 32];
+  __shared__ uint32_t before;
+  uint32_t v = 0;
+  for (uint32_t k = threadIdx.x; k < blockIdx.x; k += kScanThreads) v += sums[k];
+  v = __reduce_add_sync(0xffffffffu, v);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t t = 0;
+    for (int w = 0; w < kScanThreads / 32; ++w) t += part[w];
+    before = t;
+    if (blockIdx.x == gridDim.x - 1) start[len] = t + sums[blockIdx.x];
+  }
+  __syncthreads();
+  const uint32_t off = before;
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) {
+    const uint32_t idx = blockIdx.x * kScanTile + k * kScanThreads + threadIdx.x;
+    if (idx < len) start[idx] += off;
+  }
+}
+
+// Phases 2 and 3 of a scan of `len` entries in `ntiles` tiles.
+void scan_finish(uint32_t* start, uint32_t len, uint32_t* sums, uint32_t ntiles,
+                 cudaStream_t st) {
+  if (ntiles <= kFinishTiles) {
+    k_scan_finish<<<ntiles, kScanThreads, 0, st>>>(start, len, sums);
+    return;
+  }
+  k_scan_sums<<<1, 1024, 0, st>>>(sums, ntiles, start, len);
+  k_scan_add<<<(len + 255) / 256, 256, 0, st>>>(start, len, sums);
+}
+inline int scan_kernels(uint32_t ntiles) { return ntiles <= kFinishTiles ? 2 : 3; }
+
 __global__ void k_scatter(const uint32_t* __restrict__ cell, const uint32_t* __restrict__ rank,
                           const uint32_t* __restrict__ start, uint32_t n, uint32_t ncells,
                           uint32_t* __restrict__ perm) {
@@ -139,102 +182,88 @@ __global__ void k_scatter(const uint32_t* __restrict__ cell, const uint32_t* __r
 // Sorts every bucket's members by original index: one thread per cell,
 // insertion sort in a local array (buckets hold ~8 particles at rest
 // density and at most max_num_particles_per_cell = 64 without a
-// cell-overflow report).  Larger cells are left to k_order_crowded.  The
-// tail bucket of out-of-grid particles is left in arrival order.
+// cell-overflow report).  Cells above kOrderLocal members (an overflow the
+// sort reports, but whose outputs are still written in canonical order) are
+// left to the block's threads together: a bitonic sort in shared memory for up
+// to kCrowdedSmem members (indices are distinct, so the order is total), and
+// beyond that one thread sorts in place (a degenerate pile of thousands of
+// particles in one cell).  The tail bucket of out-of-grid particles is left
+// in arrival order.
 constexpr uint32_t kOrderLocal = 64;
-
-__global__ void k_order_cells(const uint32_t* __restrict__ start, uint32_t ncells,
-                              uint32_t* __restrict__ perm) {
-  uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncells) return;
-  const uint32_t b = start[c], e = start[c + 1];
-  if (e - b < 2 || e - b > kOrderLocal) return;
-  uint32_t a[kOrderLocal];
-  const uint32_t m = e - b;
-  for (uint32_t k = 0; k < m; ++k) {
-    uint32_t v = perm[b + k];
-    uint32_t j = k;
-    while (j > 0 && a[j - 1] > v) {
-      a[j] = a[j - 1];
-      --j;
-    }
-    a[j] = v;
-  }
-  for (uint32_t k = 0; k < m; ++k) perm[b + k] = a[k];
-}
-
-// Cells above kOrderLocal members (an overflow the sort reports, but whose
-// outputs are still written in canonical order): each block walks the cells
-// in chunks of its width, and sorts each crowded cell it finds with all its
-// threads, by a bitonic sort in shared memory for up to kCrowdedSmem
-// members (indices are distinct, so the order is total).  Beyond that one
-// thread sorts in place (a degenerate pile of thousands of particles in one
-// cell).
-constexpr uint32_t kCrowdedThreads = 256;
+constexpr uint32_t kOrderThreads = 256;
 constexpr uint32_t kCrowdedSmem = 4096;
-constexpr uint32_t kCrowdedBlocks = 256;
 
-__global__ void __launch_bounds__(kCrowdedThreads)
-    k_order_crowded(const uint32_t* __restrict__ start, uint32_t ncells,
-                    uint32_t* __restrict__ perm) {
+__global__ void __launch_bounds__(kOrderThreads)
+    k_order_cells(const uint32_t* __restrict__ start, uint32_t ncells,
+                  uint32_t* __restrict__ perm) {
   __shared__ uint32_t v[kCrowdedSmem];
-  __shared__ uint32_t crowded[kCrowdedThreads];
+  __shared__ uint32_t crowded[kOrderThreads];
   __shared__ uint32_t ncrowded;
-  for (uint32_t base = blockIdx.x * kCrowdedThreads; base < ncells;
-       base += gridDim.x * kCrowdedThreads) {
-    if (threadIdx.x == 0) ncrowded = 0;
-    __syncthreads();
-    const uint32_t c = base + threadIdx.x;
-    if (c < ncells && start[c + 1] - start[c] > kOrderLocal)
-      crowded[atomicAdd(&ncrowded, 1u)] = c;
-    __syncthreads();
-    const uint32_t nc = ncrowded;
-    for (uint32_t q = 0; q < nc; ++q) {
-      const uint32_t cc = crowded[q];
-      const uint32_t b = start[cc], m = start[cc + 1] - b;
-      if (m <= kCrowdedSmem) {
-        uint32_t len = 1;
-        while (len < m) len <<= 1;
-        for (uint32_t k = threadIdx.x; k < len; k += kCrowdedThreads)
-          v[k] = k < m ? perm[b + k] : 0xffffffffu;
-        __syncthreads();
-        for (uint32_t size = 2; size <= len; size <<= 1) {
-          for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            for (uint32_t k = threadIdx.x; k < len; k += kCrowdedThreads) {
-              const uint32_t partner = k ^ stride;
-              if (partner > k) {
-                const bool up = (k & size) == 0;
-                const uint32_t x = v[k], y = v[partner];
-                if ((x > y) == up) {
-                  v[k] = y;
-                  v[partner] = x;
-                }
+  const uint32_t c = blockIdx.x * kOrderThreads + threadIdx.x;
+  const uint32_t first = c < ncells ? start[c] : 0u;
+  const uint32_t size = c < ncells ? start[c + 1] - first : 0u;
+  if (size >= 2 && size <= kOrderLocal) {
+    uint32_t a[kOrderLocal];
+    for (uint32_t k = 0; k < size; ++k) {
+      const uint32_t x = perm[first + k];
+      uint32_t j = k;
+      while (j > 0 && a[j - 1] > x) {
+        a[j] = a[j - 1];
+        --j;
+      }
+      a[j] = x;
+    }
+    for (uint32_t k = 0; k < size; ++k) perm[first + k] = a[k];
+  }
+  if (!__syncthreads_or(size > kOrderLocal)) return;
+  if (threadIdx.x == 0) ncrowded = 0;
+  __syncthreads();
+  if (size > kOrderLocal) crowded[atomicAdd(&ncrowded, 1u)] = c;
+  __syncthreads();
+  const uint32_t nc = ncrowded;
+  for (uint32_t q = 0; q < nc; ++q) {
+    const uint32_t cc = crowded[q];
+    const uint32_t b = start[cc], m = start[cc + 1] - b;
+    if (m <= kCrowdedSmem) {
+      uint32_t len = 1;
+      while (len < m) len <<= 1;
+      for (uint32_t k = threadIdx.x; k < len; k += kOrderThreads)
+        v[k] = k < m ? perm[b + k] : 0xffffffffu;
+      __syncthreads();
+      for (uint32_t width = 2; width <= len; width <<= 1) {
+        for (uint32_t stride = width >> 1; stride > 0; stride >>= 1) {
+          for (uint32_t k = threadIdx.x; k < len; k += kOrderThreads) {
+            const uint32_t partner = k ^ stride;
+            if (partner > k) {
+              const bool up = (k & width) == 0;
+              const uint32_t x = v[k], y = v[partner];
+              if ((x > y) == up) {
+                v[k] = y;
+                v[partner] = x;
               }
             }
-            __syncthreads();
           }
-        }
-        for (uint32_t k = threadIdx.x; k < m; k += kCrowdedThreads) perm[b + k] = v[k];
-        __syncthreads();
-      } else if (threadIdx.x == 0) {
-        for (uint32_t k = b + 1; k < b + m; ++k) {
-          const uint32_t x = perm[k];
-          uint32_t j = k;
-          while (j > b && perm[j - 1] > x) {
-            perm[j] = perm[j - 1];
-            --j;
-          }
-          perm[j] = x;
+          __syncthreads();
         }
       }
-      __syncthreads();
+      for (uint32_t k = threadIdx.x; k < m; k += kOrderThreads) perm[b + k] = v[k];
+    } else if (threadIdx.x == 0) {
+      for (uint32_t k = b + 1; k < b + m; ++k) {
+        const uint32_t x = perm[k];
+        uint32_t j = k;
+        while (j > b && perm[j - 1] > x) {
+          perm[j] = perm[j - 1];
+          --j;
+        }
+        perm[j] = x;
+      }
     }
+    __syncthreads();
   }
 }
 
-inline uint32_t crowded_blocks(uint32_t ncells) {
-  const uint32_t chunks = (ncells + kCrowdedThreads - 1) / kCrowdedThreads;
-  return chunks < kCrowdedBlocks ? (chunks ? chunks : 1u) : kCrowdedBlocks;
+inline uint32_t order_blocks(uint32_t ncells) {
+  return ncells ? (ncells + kOrderThreads - 1) / kOrderThreads : 1u;
 }
 
 template <class TF>
@@ -309,8 +338,7 @@ int scan_with_flags(al_engine* e, const uint32_t* count, uint32_t* start, uint32
   uint32_t* sums = nullptr;
   ALB_TRY(e->buf("scan.sums", ntiles, &sums));
   k_scan_tiles<<<ntiles, kScanThreads, 0, st>>>(count, start, len, sums, ncells, cap, flags);
-  k_scan_sums<<<1, 1024, 0, st>>>(sums, ntiles, start, len);
-  if (ntiles > 1) k_scan_add<<<blocks_for(len, 256), 256, 0, st>>>(start, len, sums);
+  scan_finish(start, len, sums, ntiles, st);
   ALB_CUDA(cudaGetLastError());
   return AL_OK;
 }
@@ -318,7 +346,8 @@ int scan_with_flags(al_engine* e, const uint32_t* count, uint32_t* start, uint32
 
 template <class TF>
 int grid_build(al_engine* e, const Cn<TF>& c, const GridDims& g, const TF* particle_x,
-               uint32_t n, vec4<TF>* xs, uint32_t* flags, GridState& gs, cudaStream_t st) {
+               uint32_t n, vec4<TF>* xs, uint32_t* flags, GridState& gs, cudaStream_t st,
+               uint32_t* zeroed_count) {
   gs.n = n;
   gs.ncells = g.ncells;
   gs.flags = flags;
@@ -326,9 +355,11 @@ int grid_build(al_engine* e, const Cn<TF>& c, const GridDims& g, const TF* parti
   ALB_TRY(e->buf("grid.cell", n, &gs.cell));
   ALB_TRY(e->buf("grid.rank", n, &rank));
   ALB_TRY(e->buf("grid.perm", n, &gs.perm));
-  ALB_TRY(e->buf("grid.count", size_t(g.ncells) + 1, &gs.count));
+  gs.count = zeroed_count;
+  if (!zeroed_count) ALB_TRY(e->buf("grid.count", size_t(g.ncells) + 1, &gs.count));
   ALB_TRY(e->buf("grid.start", size_t(g.ncells) + 2, &gs.cell_start));
-  ALB_CUDA(cudaMemsetAsync(gs.count, 0, (size_t(g.ncells) + 1) * sizeof(uint32_t), st));
+  if (!zeroed_count)
+    ALB_CUDA(cudaMemsetAsync(gs.count, 0, (size_t(g.ncells) + 1) * sizeof(uint32_t), st));
   if (n == 0) {
     ALB_CUDA(cudaMemsetAsync(gs.cell_start, 0, (size_t(g.ncells) + 2) * sizeof(uint32_t), st));
     return AL_OK;
@@ -339,11 +370,9 @@ int grid_build(al_engine* e, const Cn<TF>& c, const GridDims& g, const TF* parti
                           st));
   k_scatter<<<blocks_for(n, kBlock), kBlock, 0, st>>>(gs.cell, rank, gs.cell_start, n, g.ncells,
                                                       gs.perm);
-  k_order_cells<<<blocks_for(g.ncells, kBlock), kBlock, 0, st>>>(gs.cell_start, g.ncells,
+  k_order_cells<<<order_blocks(g.ncells), kOrderThreads, 0, st>>>(gs.cell_start, g.ncells,
                                                                  gs.perm);
-  k_order_crowded<<<crowded_blocks(g.ncells), kCrowdedThreads, 0, st>>>(gs.cell_start, g.ncells,
-                                                                        gs.perm);
-  k_gather_x<TF><<<blocks_for(n, kBlock), kBlock, 0, st>>>(particle_x, gs.perm, n, xs);
+  if (xs) k_gather_x<TF><<<blocks_for(n, kBlock), kBlock, 0, st>>>(particle_x, gs.perm, n, xs);
   ALB_CUDA(cudaGetLastError());
   return AL_OK;
 }
@@ -369,15 +398,17 @@ int grid_build_fused(al_engine* e, TF h, const uint32_t* blk_scene, const SortSc
   ALB_TRY(scan_with_flags(e, gs.count, gs.cell_start, ncells + 1, 0u, 0u, nullptr, st));
   k_scatter_fused<<<blocks_for(narena, kBlock), kBlock, 0, st>>>(gs.cell, rank, gs.cell_start,
                                                                 narena, gs.perm);
-  k_order_cells<<<blocks_for(ncells, kBlock), kBlock, 0, st>>>(gs.cell_start, ncells, gs.perm);
-  k_order_crowded<<<crowded_blocks(ncells), kCrowdedThreads, 0, st>>>(gs.cell_start, ncells,
-                                                                      gs.perm);
+  k_order_cells<<<order_blocks(ncells), kOrderThreads, 0, st>>>(gs.cell_start, ncells, gs.perm);
   ALB_CUDA(cudaGetLastError());
   return AL_OK;
 }
 
+// pad counts, hash, scan, scatter, order
 uint32_t grid_fused_kernels(uint32_t ncells) {
-  return 7u + (grid_scan_tiles(ncells + 1) > 1 ? 1u : 0u);
+  return 4u + uint32_t(scan_kernels(grid_scan_tiles(ncells + 1)));
+}
+int grid_build_kernels(uint32_t ncells, bool gather) {
+  return 3 + scan_kernels(grid_scan_tiles(ncells + 1)) + (gather ? 1 : 0);
 }
 
 uint32_t grid_scan_tiles(uint32_t len) { return (len + kScanTile - 1) / kScanTile; }
@@ -397,12 +428,10 @@ int grid_sort_into(const Cn<TF>& c, const GridDims& g, const TF* particle_x, uin
   const uint32_t ntiles = grid_scan_tiles(len);
   k_scan_tiles<<<ntiles, kScanThreads, 0, st>>>(sc.count, sc.start, len, sc.sums, g.ncells,
                                                  g.cap_cell, sc.flags);
-  k_scan_sums<<<1, 1024, 0, st>>>(sc.sums, ntiles, sc.start, len);
-  if (ntiles > 1) k_scan_add<<<blocks_for(len, 256), 256, 0, st>>>(sc.start, len, sc.sums);
+  scan_finish(sc.start, len, sc.sums, ntiles, st);
   k_scatter<<<blocks_for(n, kBlock), kBlock, 0, st>>>(cell, sc.rank, sc.start, n, g.ncells,
                                                       perm);
-  k_order_cells<<<blocks_for(g.ncells, kBlock), kBlock, 0, st>>>(sc.start, g.ncells, perm);
-  k_order_crowded<<<crowded_blocks(g.ncells), kCrowdedThreads, 0, st>>>(sc.start, g.ncells, perm);
+  k_order_cells<<<order_blocks(g.ncells), kOrderThreads, 0, st>>>(sc.start, g.ncells, perm);
   ALB_CUDA(cudaGetLastError());
   return AL_OK;
 }
@@ -416,8 +445,9 @@ template int grid_build_fused<float>(al_engine*, float, const uint32_t*,
                                      const SortScene<float>*, uint32_t, uint32_t, uint32_t,
                                      GridState&, cudaStream_t);
 template int grid_build<float>(al_engine*, const Cn<float>&, const GridDims&, const float*,
-                               uint32_t, vec4<float>*, uint32_t*, GridState&, cudaStream_t);
+                               uint32_t, vec4<float>*, uint32_t*, GridState&, cudaStream_t, uint32_t*);
 template int grid_build<double>(al_engine*, const Cn<double>&, const GridDims&, const double*,
-                                uint32_t, vec4<double>*, uint32_t*, GridState&, cudaStream_t);
+                                uint32_t, vec4<double>*, uint32_t*, GridState&, cudaStream_t,
+                                uint32_t*);
 
 }  // namespace alb

@@ -4,7 +4,7 @@
 // appends particles to fixed-capacity buckets in atomicAdd order; the engine
 // builds a compact cell-sorted permutation in canonical (cell, index) order:
 //   1. hash:    cell id per particle, arrival rank within the cell
-//   2. scan:    exclusive prefix sum of cell counts (3 passes, no waits)
+//   2. scan:    exclusive prefix sum of cell counts (2 or 3 passes, no waits)
 //   3. scatter: slot = cell_start + arrival rank
 //   4. order:   each cell's members sorted by original index (makes the
 //               permutation independent of atomic arrival order)
@@ -26,16 +26,19 @@ struct GridState {
   uint32_t* flags = nullptr;       // [4] grid_anomaly[0..2] + spare (device)
 };
 
-// Kernels one grid_build launches (hash, three scan passes, scatter, the two
-// per-cell orderings, gather).
-constexpr int kGridBuildKernels = 8;
+// Kernels one grid_build launches (hash, scan, scatter, the per-cell ordering
+// and, with `gather`, the positions).
+int grid_build_kernels(uint32_t ncells, bool gather = true);
 
-// Hashes, sorts and gathers positions into `xs` (sorted order, w = 0).
-// particle_x is the caller's [n][3] array.  `flags` must be zeroed by the
-// caller (it is also used by later passes).
+// Hashes, sorts and gathers positions into `xs` (sorted order, w = 0; null:
+// no gather).  particle_x is the caller's [n][3] array.  `flags` must be zeroed
+// by the caller (it is also used by later passes).  `zeroed_count`: the
+// caller's buffer of ncells + 1 zeros to count in (null: the engine's own,
+// cleared here).
 template <class TF>
 int grid_build(al_engine* e, const Cn<TF>& c, const GridDims& g, const TF* particle_x,
-               uint32_t n, vec4<TF>* xs, uint32_t* flags, GridState& gs, cudaStream_t st);
+               uint32_t n, vec4<TF>* xs, uint32_t* flags, GridState& gs, cudaStream_t st,
+               uint32_t* zeroed_count = nullptr);
 
 // One scene of a fused batch's sort: its positions (the caller's [n][3]),
 // grid, first cell in the batch's concatenated cells (its ncells cells, then

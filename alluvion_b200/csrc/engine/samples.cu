@@ -585,7 +585,7 @@ int sample_fluid(al_engine* engine, const typename SampleTypes<TF>::cn* cn, cons
   ALB_TRY(engine->buf("flags", 4, &sflags));
   ALB_CUDA(cudaMemsetAsync(sflags, 0, 4 * sizeof(uint32_t), st));
   GridState ss;
-  ALB_LAUNCH(engine, "sample_sort", kGridBuildKernels, st,
+  ALB_LAUNCH(engine, "sample_sort", grid_build_kernels(g.ncells), st,
              ALB_TRY(grid_build<TF>(engine, c, g, req->sample_x, req->num_samples, sxs, sflags,
                                     ss, st)));
   engine->ns = "sample.";
@@ -617,7 +617,7 @@ int sample_fluid(al_engine* engine, const typename SampleTypes<TF>::cn* cn, cons
     grid_x = all;
   }
   GridState gs;
-  ALB_LAUNCH(engine, "sample_grid", kGridBuildKernels, st,
+  ALB_LAUNCH(engine, "sample_grid", grid_build_kernels(g.ncells), st,
              ALB_TRY(grid_build<TF>(engine, c, g, grid_x, npts, xs, flags, gs, st)));
   SampleDev<TF> sd{req->sample_x,
                    req->num_samples,

@@ -235,8 +235,8 @@ struct LoadXV {
 
 // Visits the lane's neighbors in list order.  A list is stored in groups of
 // kNbrGroup entries, one 16-byte load each; lane `sub` takes groups sub,
-// sub + tpp, ...  Each round loads the groups of B entries, then gathers
-// `load(t)` of the B entries, then runs `f(t, loaded)` for each.  The
+// sub + tpp, ... and gathers `load(t)` of B entries, then runs `f(t, loaded)`
+// for each.  The
 // entries that pad a list's last group name the particle itself: every pass
 // weighs its neighbors by grad W, which is exactly zero there.  At one thread
 // per particle that is the order of a plain loop over the list; with tpp > 1
@@ -251,39 +251,50 @@ struct LoadXV {
 template <int B, class TF, class Load, class F>
 __device__ __forceinline__ void for_each_neighbor(const StepState<TF>& S, const Lane& L,
                                                   uint32_t cnt, Load&& load, F&& f) {
-  constexpr int kG = B > 4 ? B / 4 : 1;  // groups per round
-  constexpr int kE = B < 4 ? B : 4;      // entries gathered together per group
-  static_assert(kNbrGroup == 4 && (B % 4 == 0 || 4 % B == 0), "rounds of whole groups");
-  const uint4* list = reinterpret_cast<const uint4*>(S.nbr) + L.s;
-  const uint32_t ng = (cnt + kNbrGroup - 1) / kNbrGroup;
-  for (uint32_t g0 = L.sub; g0 < ng; g0 += kG * L.tpp) {
-    uint32_t t[4 * kG];
-#pragma unroll
-    for (int u = 0; u < kG; ++u) {
-      const uint32_t g = g0 + u * L.tpp;
-      uint4 q{L.s, L.s, L.s, L.s};
-      if (u == 0 || g < ng) q = __ldcs(list + size_t(g) * S.ls);
-      t[4 * u] = q.x;
-      t[4 * u + 1] = q.y;
-      t[4 * u + 2] = q.z;
-      t[4 * u + 3] = q.w;
+  // entries a lane takes at a time: a group, or in double, whose passes are
+  // bound by arithmetic, half of one, which splits a list more evenly
+  constexpr uint32_t kU = sizeof(TF) == 4 ? kNbrGroup : kNbrGroup / 2;
+  constexpr int kE = B < int(kU) ? B : int(kU);  // entries gathered together
+  static_assert(kNbrGroup == 4 && kU % kE == 0, "rounds of whole units");
+  const uint32_t* list = S.nbr + size_t(L.s) * kNbrGroup;
+  for (uint32_t k = L.sub * kU; k < cnt; k += kU * L.tpp) {
+    const uint32_t* p = list + size_t(k / kNbrGroup) * S.ls * kNbrGroup + k % kNbrGroup;
+    uint32_t t[kU];
+    if constexpr (kU == 4) {
+      const uint4 q = __ldcs(reinterpret_cast<const uint4*>(p));
+      t[0] = q.x;
+      t[1] = q.y;
+      t[2] = q.z;
+      t[3] = q.w;
+    } else {
+      const uint2 q = __ldcs(reinterpret_cast<const uint2*>(p));
+      t[0] = q.x;
+      t[1] = q.y;
     }
 #pragma unroll
-    for (int h = 0; h < 4 * kG; h += kE * kG) {
-      decltype(load(0u)) r[kE * kG];
+    for (uint32_t h = 0; h < kU; h += kE) {
+      decltype(load(0u)) r[kE];
 #pragma unroll
-      for (int b = 0; b < kE * kG; ++b) r[b] = load(t[h + b]);
+      for (int b = 0; b < kE; ++b) r[b] = load(t[h + b]);
 #pragma unroll
-      for (int b = 0; b < kE * kG; ++b) f(t[h + b], r[b]);
+      for (int b = 0; b < kE; ++b) f(t[h + b], r[b]);
     }
   }
 }
 
 // Records a velocity-divergence pass gathers together: four float ones, two
-// with the periodic wrap or in double, whose records are 64 bytes.
+// with the periodic wrap or in double, whose records are 64 bytes.  The
+// compiler's own register counts are the best for float passes (32; held to
+// that number by hand the pass slowed from 757 to 890 us at 8,388,608
+// particles); beside the wrap it takes 45, and 40 are faster (29.2 instead of
+// 34.5 us at 209,040 particles).
 template <class TF, bool WR>
 constexpr int xv_batch() {
   return sizeof(TF) == 4 && !WR ? 4 : 2;
+}
+template <class TF, bool WR, bool BT>
+constexpr int divergence_blocks() {  // least resident kMaxBlock-thread blocks (0: open)
+  return sizeof(TF) == 8 ? 4 : WR && !BT ? 6 : 0;
 }
 
 // Sum over neighbors of V (v_i - v_j) . grad W_ij plus the boundary terms
@@ -336,12 +347,14 @@ __device__ __forceinline__ TF density_adv(const Cn<TF>& c, const StepState<TF>& 
 }
 
 // ------------------------------------------------------------- kernels
-// With BT every scene of a fused batch in one launch: the block's scene's
-// buffers (S.io; S.perm holds arena slots s0 + i), the sorted positions
-// gathered here too.
+// The caller's state in sorted order; a one-scene launch also initialises the
+// step's control block.  With BT every scene of a fused batch in one launch:
+// the block's scene's buffers (S.io; S.perm holds arena slots s0 + i).
 template <class TF, bool DF, bool BT = false>
-__global__ void k_gather_state(StepState<TF> S, const TF* __restrict__ v_ref,
-                               const TF* __restrict__ k_ref, const TF* __restrict__ kv_ref) {
+__global__ void k_gather_state(StepState<TF> S, const TF* __restrict__ x_ref,
+                               const TF* __restrict__ v_ref, const TF* __restrict__ k_ref,
+                               const TF* __restrict__ kv_ref) {
+  if (!BT && blockIdx.x == 0) step_init(S);
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   BlockSpan B;
   if (!block_scene<BT>(S, B) || s >= B.end) return;
@@ -352,13 +365,13 @@ __global__ void k_gather_state(StepState<TF> S, const TF* __restrict__ v_ref,
     v_ref = io.v_in;
     k_ref = io.kappa_in;
     kv_ref = io.kappa_v_in;
-    const vec3<TF> p = ld3(io.x_in, i);
-    S.x[s] = vec4<TF>{p.x, p.y, p.z, TF(0)};
+    x_ref = io.x_in;
   } else {
     i = S.perm[s];
   }
-  const vec3<TF> v = ld3(v_ref, i);
-  RX(S, s) = vec4<TF>{S.x[s].x, S.x[s].y, S.x[s].z, TF(0)};
+  const vec3<TF> p = ld3(x_ref, i), v = ld3(v_ref, i);
+  S.x[s] = vec4<TF>{p.x, p.y, p.z, TF(0)};
+  RX(S, s) = vec4<TF>{p.x, p.y, p.z, TF(0)};
   RV(S, s) = vec4<TF>{v.x, v.y, v.z, TF(0)};  // rho follows from the build
   S.kappa[s] = k_ref ? k_ref[i] : TF(0);
   if (DF) S.kappa_v[s] = kv_ref ? kv_ref[i] : TF(0);
@@ -545,7 +558,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_kappa(Cn<TF> c, StepState<TF> S) 
 // compute_velocity_of_density_change (runner.hpp:3297-3314); also forms
 // k = rho_adv * alpha for the first divergence iteration.
 template <class TF, bool WR = false, bool BT = false>
-__global__ void __launch_bounds__(kMaxBlock) k_df_rho_adv_init(Cn<TF> c, StepState<TF> S) {
+__global__ void __launch_bounds__(kMaxBlock, (divergence_blocks<TF, WR, BT>()))
+    k_df_rho_adv_init(Cn<TF> c, StepState<TF> S, cudaGraphConditionalHandle handle,
+                      int use_handle) {
+  if (!BT && blockIdx.x == 0 && threadIdx.x == 0) loop_begin(*S.ctrl, 0, handle, use_handle);
   if constexpr (!WR) c.wrap = 0;  // non-periodic: the wrap branches fold away
   BlockSpan B;
   if (!block_scene<BT>(S, B)) return;
@@ -563,7 +579,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_df_rho_adv_init(Cn<TF> c, StepSta
 // compute_divergence_solve_density_error (runner.hpp:3396-3410) with the
 // mean of solver_df.hpp:160-161 reduced in double on the device.
 template <class TF, bool WR = false, bool BT = false>
-__global__ void __launch_bounds__(kMaxBlock)
+__global__ void __launch_bounds__(kMaxBlock, (divergence_blocks<TF, WR, BT>()))
     k_df_residual(Cn<TF> c, StepState<TF> S, cudaGraphConditionalHandle handle, int use_handle) {
   if constexpr (!WR) c.wrap = 0;  // non-periodic: the wrap branches fold away
   BlockSpan B;
@@ -720,7 +736,7 @@ __global__ void k_integrate_np(StepState<TF> S) {
 // previous-step value under the same gate (rho_adv > 1), unless the floor
 // gate is set.
 template <class TF, bool WR = false, bool BT = false>
-__global__ void __launch_bounds__(kMaxBlock)
+__global__ void __launch_bounds__(kMaxBlock, (divergence_blocks<TF, WR, BT>()))
     k_p_warm0(Cn<TF> c, StepState<TF> S, const float* __restrict__ pred,
               const uint32_t* __restrict__ floor) {
   if constexpr (!WR) c.wrap = 0;  // non-periodic: the wrap branches fold away
@@ -742,7 +758,10 @@ __global__ void __launch_bounds__(kMaxBlock)
 
 // compute_rho_adv (runner.hpp:3525-3541); also k for the first iteration.
 template <class TF, bool WR = false, bool BT = false>
-__global__ void __launch_bounds__(kMaxBlock) k_p_rho_adv_init(Cn<TF> c, StepState<TF> S) {
+__global__ void __launch_bounds__(kMaxBlock, (divergence_blocks<TF, WR, BT>()))
+    k_p_rho_adv_init(Cn<TF> c, StepState<TF> S, cudaGraphConditionalHandle handle,
+                     int use_handle) {
+  if (!BT && blockIdx.x == 0 && threadIdx.x == 0) loop_begin(*S.ctrl, 1, handle, use_handle);
   if constexpr (!WR) c.wrap = 0;  // non-periodic: the wrap branches fold away
   BlockSpan B;
   if (!block_scene<BT>(S, B)) return;
@@ -760,7 +779,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_p_rho_adv_init(Cn<TF> c, StepStat
 // compute_pressure_solve_density_error (runner.hpp:3590-3604); the mean is
 // sum(rho_adv - 1) / N in double (solver_df.hpp:323-325 forms sum/N - 1).
 template <class TF, bool WR = false, bool BT = false>
-__global__ void __launch_bounds__(kMaxBlock)
+__global__ void __launch_bounds__(kMaxBlock, (divergence_blocks<TF, WR, BT>()))
     k_p_residual(Cn<TF> c, StepState<TF> S, cudaGraphConditionalHandle handle, int use_handle) {
   if constexpr (!WR) c.wrap = 0;  // non-periodic: the wrap branches fold away
   BlockSpan B;
@@ -868,7 +887,9 @@ __global__ void __launch_bounds__(kMaxBlock) k_ii_predict0(Cn<TF> c, StepState<T
 
 // predict_advection1 (runner.hpp:2640-2690).  aii goes to kk.
 template <class TF, bool WR = false>
-__global__ void __launch_bounds__(kMaxBlock) k_ii_predict1(Cn<TF> c, StepState<TF> S) {
+__global__ void __launch_bounds__(kMaxBlock)
+    k_ii_predict1(Cn<TF> c, StepState<TF> S, cudaGraphConditionalHandle handle, int use_handle) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) loop_begin(*S.ctrl, 1, handle, use_handle);
   if constexpr (!WR) c.wrap = 0;  // non-periodic: the wrap branches fold away
   const Lane L = pair_lane(S);
   const TF dt = S.ctrl->dt;
@@ -1076,7 +1097,9 @@ __global__ void __launch_bounds__(kMaxBlock) k_i_advect(StepState<TF> S) {
 // calculate_isph_diagonal_adv_density (runner.hpp:2901-2954): the Jacobi
 // diagonal (times rho0) into kk, the advected density into rho_adv.
 template <class TF, bool WR = false>
-__global__ void __launch_bounds__(kMaxBlock) k_i_diag(Cn<TF> c, StepState<TF> S) {
+__global__ void __launch_bounds__(kMaxBlock)
+    k_i_diag(Cn<TF> c, StepState<TF> S, cudaGraphConditionalHandle handle, int use_handle) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) loop_begin(*S.ctrl, 1, handle, use_handle);
   if constexpr (!WR) c.wrap = 0;  // non-periodic: the wrap branches fold away
   const Lane L = pair_lane(S);
   const TF dt = S.ctrl->dt;
@@ -1278,6 +1301,10 @@ struct StepPlan {
   StepState<TF> S;
   uint32_t* flags = nullptr;
   BodyDev<TF>* bodies_dev = nullptr;
+  // cell counts, then the rigid slots: cleared together
+  char* zeroed = nullptr;
+  size_t zeroed_bytes = 0;
+  uint32_t* zeroed_count = nullptr;
   Staging<TF> io;
   // learned warm start (float DFSPH steps): features in sorted order and
   // the network's predictions; features_out in original order
@@ -1401,20 +1428,16 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
   const uint32_t n = S.n, nb = S.nb;
   const bool iisph = P.iisph, div = P.div, den = P.den;
   const bool wr = c.wrap != 0;  // periodic-y instantiations of the pair passes
-  ALB_CUDA(cudaMemcpyAsync(S.ctrl, P.io.hc, sizeof(Ctrl<TF>), cudaMemcpyHostToDevice, st));
-  if (nb) {
-    ALB_CUDA(cudaMemcpyAsync(P.bodies_dev, P.io.hb, sizeof(BodyDev<TF>) * nb,
-                             cudaMemcpyHostToDevice, st));
-    ALB_CUDA(cudaMemcpyAsync(S.rigid, P.io.hr, sizeof(RigidDev<TF>) * nb, cudaMemcpyHostToDevice,
-                             st));
-  }
-  ALB_CUDA(cudaMemsetAsync(P.flags, 0, 4 * sizeof(uint32_t), st));
-  ALB_CUDA(cudaMemsetAsync(S.ft, 0, size_t(S.grid) * (nb ? nb : 1) * 6 * sizeof(double), st));
-  ALB_LAUNCH(e, "step_init", 1, st, k_step_init<TF><<<1, 32, 0, st>>>(S));
+  // control block, bodies, rigid state and cleared anomaly flags in one copy
+  using SL = StagingLayout<TF>;
+  ALB_CUDA(cudaMemcpyAsync(S.ctrl, P.io.hc, SL::bytes, cudaMemcpyHostToDevice, st));
+  // the cell counts and the rigid slots behind them
+  ALB_CUDA(cudaMemsetAsync(P.zeroed, 0, P.zeroed_bytes, st));
   // ---- grid, boundaries, neighbors, density (+ DFSPH factor)
   GridState gs;
-  ALB_LAUNCH(e, "grid_sort", kGridBuildKernels, st,
-             ALB_TRY(grid_build<TF>(e, c, P.g, f->particle_x, n, S.x, P.flags, gs, st)));
+  ALB_LAUNCH(e, "grid_sort", grid_build_kernels(P.g.ncells, false), st,
+             ALB_TRY(grid_build<TF>(e, c, P.g, f->particle_x, n, static_cast<vec4<TF>*>(nullptr),
+                                    P.flags, gs, st, P.zeroed_count)));
   S.perm = gs.perm;
   const uint32_t blocks = blocks_for(n, kBlock);
   // grid, block and lane state of pair pass group `g` (launch-shape table)
@@ -1430,12 +1453,14 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
     const TF* kref = iisph ? f->particle_pressure : f->particle_kappa;
     if (iisph)
       ALB_LAUNCH(e, "gather_state", 1, st,
-                 k_gather_state<TF, false><<<blocks, kBlock, 0, st>>>(S, f->particle_v, kref,
-                                                                      nullptr));
+                 k_gather_state<TF, false><<<blocks, kBlock, 0, st>>>(S, f->particle_x,
+                                                                      f->particle_v, kref, nullptr));
     else
       ALB_LAUNCH(e, "gather_state", 1, st,
-                 k_gather_state<TF, true><<<blocks, kBlock, 0, st>>>(S, f->particle_v, kref,
-                                                                     f->particle_kappa_v));
+                 k_gather_state<TF, true><<<blocks, kBlock, 0, st>>>(
+                     S, f->particle_x, f->particle_v, kref, f->particle_kappa_v));
+  } else {
+    ALB_LAUNCH(e, "step_init", 1, st, k_step_init<TF><<<1, 32, 0, st>>>(S));
   }
   BoundaryState<TF> bs{nb, S.mask, S.bx, S.bk, &S.ctrl->rep.num_active_boundary_pairs, S.ls};
   if (nb)
@@ -1488,21 +1513,21 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
     ALB_LAUNCH(e, "neighbors", 1, st,
                ALB_TRY(build_neighbors_density<TF>(c, P.g, gs, S.x, sbk, S.nbr, S.ncount, S.rho,
                                                    iisph ? nullptr : S.alpha, rho_rec, st)));
-  // One solver loop: kernel `k_loop_begin` sets the first condition, `body`
-  // launches one iteration on the given stream.
-  auto solve = [&](int density_solve, uint32_t max_iter, auto&& body) -> int {
+  // One solver loop: `begin`, the pass that forms the solve's first source
+  // term, also sets the first condition (loop_begin); `body` launches one
+  // iteration on the given stream.
+  auto solve = [&](uint32_t max_iter, auto&& begin, auto&& body) -> int {
     if (capture) {
       ++*loops;
       return capture_while(
           e, st,
           [&](cudaGraphConditionalHandle h) -> int {
-            ALB_LAUNCH(e, "loop_begin", 1, st,
-                       k_loop_begin<TF><<<1, 1, 0, st>>>(S, density_solve, h, 1));
+            begin(h, 1);
             return AL_OK;
           },
           body);
     }
-    ALB_LAUNCH(e, "loop_begin", 1, st, k_loop_begin<TF><<<1, 1, 0, st>>>(S, density_solve, 0, 0));
+    begin(cudaGraphConditionalHandle(0), 0);
     bool go = max_iter > 0;
     while (go) {
       ALB_TRY(body(st, cudaGraphConditionalHandle(0), 0));
@@ -1518,13 +1543,14 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
         ALB_LAUNCH(e, "div_warm1", 1, st,
                    (wr ? k_kappa<TF, kDivWarm, true><<<pg_, pb_, 0, st>>>(c, Sg_) : k_kappa<TF, kDivWarm, false><<<pg_, pb_, 0, st>>>(c, Sg_)));
       }
-      {
-        uint32_t pg_, pb_;
-        const StepState<TF> Sg_ = pair_shape("div_rho_adv", pg_, pb_);
-        ALB_LAUNCH(e, "div_rho_adv", 1, st,
-                   (wr ? k_df_rho_adv_init<TF, true><<<pg_, pb_, 0, st>>>(c, Sg_) : k_df_rho_adv_init<TF, false><<<pg_, pb_, 0, st>>>(c, Sg_)));
-      }
-      ALB_TRY(solve(0, P.io.hc->max_div,
+      ALB_TRY(solve(P.io.hc->max_div,
+                    [&](cudaGraphConditionalHandle h, int use) {
+                      uint32_t pg_, pb_;
+                      const StepState<TF> Sg_ = pair_shape("div_rho_adv", pg_, pb_);
+                      ALB_LAUNCH(e, "div_rho_adv", 1, st,
+                                 (wr ? k_df_rho_adv_init<TF, true><<<pg_, pb_, 0, st>>>(c, Sg_, h, use)
+                                     : k_df_rho_adv_init<TF, false><<<pg_, pb_, 0, st>>>(c, Sg_, h, use)));
+                    },
                     [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) -> int {
                       {
                         uint32_t pg_, pb_;
@@ -1562,13 +1588,14 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
           ALB_LAUNCH(e, "press_warm1", 1, st,
                      (wr ? k_kappa<TF, kPressWarm, true><<<pg_, pb_, 0, st>>>(c, Sg_) : k_kappa<TF, kPressWarm, false><<<pg_, pb_, 0, st>>>(c, Sg_)));
         }
-        {
-          uint32_t pg_, pb_;
-          const StepState<TF> Sg_ = pair_shape("press_rho_adv", pg_, pb_);
-          ALB_LAUNCH(e, "press_rho_adv", 1, st,
-                     (wr ? k_p_rho_adv_init<TF, true><<<pg_, pb_, 0, st>>>(c, Sg_) : k_p_rho_adv_init<TF, false><<<pg_, pb_, 0, st>>>(c, Sg_)));
-        }
-        ALB_TRY(solve(1, P.io.hc->max_den,
+        ALB_TRY(solve(P.io.hc->max_den,
+                      [&](cudaGraphConditionalHandle h, int use) {
+                        uint32_t pg_, pb_;
+                        const StepState<TF> Sg_ = pair_shape("press_rho_adv", pg_, pb_);
+                        ALB_LAUNCH(e, "press_rho_adv", 1, st,
+                                   (wr ? k_p_rho_adv_init<TF, true><<<pg_, pb_, 0, st>>>(c, Sg_, h, use)
+                                       : k_p_rho_adv_init<TF, false><<<pg_, pb_, 0, st>>>(c, Sg_, h, use)));
+                      },
                       [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) -> int {
                         {
                           uint32_t pg_, pb_;
@@ -1595,12 +1622,14 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
                      f->particle_kappa_v, f->particle_density_adv, P.warm_floor)));
     } else if (P.isph) {
       ALB_LAUNCH(e, "i_advect", 1, st, k_i_advect<TF><<<blocks, kBlock, 0, st>>>(S));
-      {
-        uint32_t pg_, pb_;
-        const StepState<TF> Sg_ = pair_shape("i_diag", pg_, pb_);
-        ALB_LAUNCH(e, "i_diag", 1, st, (wr ? k_i_diag<TF, true><<<pg_, pb_, 0, st>>>(c, Sg_) : k_i_diag<TF, false><<<pg_, pb_, 0, st>>>(c, Sg_)));
-      }
-      ALB_TRY(solve(1, P.io.hc->max_den,
+      ALB_TRY(solve(P.io.hc->max_den,
+                    [&](cudaGraphConditionalHandle h, int use) {
+                      uint32_t pg_, pb_;
+                      const StepState<TF> Sg_ = pair_shape("i_diag", pg_, pb_);
+                      ALB_LAUNCH(e, "i_diag", 1, st,
+                                 (wr ? k_i_diag<TF, true><<<pg_, pb_, 0, st>>>(c, Sg_, h, use)
+                                     : k_i_diag<TF, false><<<pg_, pb_, 0, st>>>(c, Sg_, h, use)));
+                    },
                     [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) -> int {
                       {
                         uint32_t pg_, pb_;
@@ -1628,12 +1657,14 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
         const StepState<TF> Sg_ = pair_shape("ii_predict0", pg_, pb_);
         ALB_LAUNCH(e, "ii_predict0", 1, st, (wr ? k_ii_predict0<TF, true><<<pg_, pb_, 0, st>>>(c, Sg_) : k_ii_predict0<TF, false><<<pg_, pb_, 0, st>>>(c, Sg_)));
       }
-      {
-        uint32_t pg_, pb_;
-        const StepState<TF> Sg_ = pair_shape("ii_predict1", pg_, pb_);
-        ALB_LAUNCH(e, "ii_predict1", 1, st, (wr ? k_ii_predict1<TF, true><<<pg_, pb_, 0, st>>>(c, Sg_) : k_ii_predict1<TF, false><<<pg_, pb_, 0, st>>>(c, Sg_)));
-      }
-      ALB_TRY(solve(1, P.io.hc->max_den,
+      ALB_TRY(solve(P.io.hc->max_den,
+                    [&](cudaGraphConditionalHandle h, int use) {
+                      uint32_t pg_, pb_;
+                      const StepState<TF> Sg_ = pair_shape("ii_predict1", pg_, pb_);
+                      ALB_LAUNCH(e, "ii_predict1", 1, st,
+                                 (wr ? k_ii_predict1<TF, true><<<pg_, pb_, 0, st>>>(c, Sg_, h, use)
+                                     : k_ii_predict1<TF, false><<<pg_, pb_, 0, st>>>(c, Sg_, h, use)));
+                    },
                     [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) -> int {
                       {
                         uint32_t pg_, pb_;
@@ -1672,11 +1703,7 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
   }
   ALB_CUDA(cudaGetLastError());
   // ---- read back: report, rigid state, anomaly flags
-  ALB_CUDA(cudaMemcpyAsync(P.io.hc, S.ctrl, sizeof(Ctrl<TF>), cudaMemcpyDeviceToHost, st));
-  if (nb)
-    ALB_CUDA(cudaMemcpyAsync(P.io.hr, S.rigid, sizeof(RigidDev<TF>) * nb, cudaMemcpyDeviceToHost,
-                             st));
-  ALB_CUDA(cudaMemcpyAsync(P.io.hf, P.flags, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  ALB_CUDA(cudaMemcpyAsync(P.io.hc, S.ctrl, SL::bytes, cudaMemcpyDeviceToHost, st));
   return AL_OK;
 }
 
@@ -1810,7 +1837,19 @@ int prepare_step(al_engine* e, const StepArgs<TF>& A, StepPlan<TF>& P, uint32_t 
   if (S.grid == 0) S.grid = 1;
   // ---- buffers
   if (alloc) {
-    ALB_TRY(e->buf("flags", 4, &P.flags));
+    // the device copy of the staging slot
+    using SL = StagingLayout<TF>;
+    char* stage = nullptr;
+    ALB_TRY(e->buf("stage", SL::bytes, &stage));
+    S.ctrl = reinterpret_cast<Ctrl<TF>*>(stage);
+    P.bodies_dev = reinterpret_cast<BodyDev<TF>*>(stage + SL::bodies);
+    S.rigid = reinterpret_cast<RigidDev<TF>*>(stage + SL::rigid);
+    P.flags = reinterpret_cast<uint32_t*>(stage + SL::flag + 64);
+    const size_t count_bytes = SL::up64((size_t(P.g.ncells) + 1) * sizeof(uint32_t));
+    P.zeroed_bytes = count_bytes + size_t(nb ? S.grid : 0) * nb * 6 * sizeof(double);
+    ALB_TRY(e->buf("zeroed", P.zeroed_bytes, &P.zeroed));
+    P.zeroed_count = reinterpret_cast<uint32_t*>(P.zeroed);
+    S.ft = reinterpret_cast<double*>(P.zeroed + count_bytes);
     ALB_TRY(e->buf("sorted.x", size_t(n) + kSortedPad, &S.x));
     ALB_TRY(e->buf("sorted.rec", size_t(n) * 2, &S.rec));
     ALB_TRY(e->buf("sorted.a", n, &S.a));
@@ -1836,12 +1875,8 @@ int prepare_step(al_engine* e, const StepArgs<TF>& A, StepPlan<TF>& P, uint32_t 
     ALB_TRY(e->buf("bnd.mask", n, &S.mask));
     ALB_TRY(e->buf("bnd.x", size_t(nb ? nb : 1) * n, &S.bx));
     ALB_TRY(e->buf("bnd.k", size_t(nb ? nb : 1) * n, &S.bk));
-    ALB_TRY(e->buf("bodies", nb ? nb : 1, &P.bodies_dev));
-    ALB_TRY(e->buf("rigid", nb ? nb : 1, &S.rigid));
-    ALB_TRY(e->buf("ft", size_t(S.grid) * (nb ? nb : 1) * 6, &S.ft));
     ALB_TRY(e->buf("ftp", size_t(kRigidChunks) * (nb ? nb : 1) * 6, &P.ftp));
     ALB_TRY(e->buf("red", S.grid, &S.red));
-    ALB_TRY(e->buf("ctrl", 1, &S.ctrl));
   }
   S.bodies = P.bodies_dev;
   const al_warm_start* warm = A.warm;
@@ -1885,6 +1920,7 @@ int prepare_step(al_engine* e, const StepArgs<TF>& A, StepPlan<TF>& P, uint32_t 
   hc->max_den = sp->max_density_solve;
   hc->integrate_rigids = sp->integrate_rigids;
   for (int k = 0; k < 3; ++k) hc->pile_gravity[k] = TF(sp->pile_gravity[k]);
+  for (int k = 0; k < 4; ++k) P.io.hf[k] = 0;
   for (uint32_t b = 0; b < nb; ++b) {
     P.io.hb[b] = to_body_dev<TF>(A.bodies[b]);
     ALB_TRY(validate_body(P.io.hb[b], true, true));
@@ -2383,7 +2419,7 @@ int enqueue_fused_head(al_engine* e, const StepPlan<TF>& P0, FusedPlan<TF>& F, c
   const StepState<TF>& S = F.S;
   const uint32_t G = F.nblocks, B = kFusedBlock;
   ALB_LAUNCH(e, "gather_state", 1, st,
-             (k_gather_state<TF, true, true><<<G, B, 0, st>>>(S, nullptr, nullptr, nullptr)));
+             (k_gather_state<TF, true, true><<<G, B, 0, st>>>(S, nullptr, nullptr, nullptr, nullptr)));
   ALB_LAUNCH(e, "boundary", 1, st,
              ALB_TRY(sample_boundaries_fused<TF>(c, S.x, F.N, S.blk_scene, F.bnd, F.K, G, S.mask,
                                                  S.bx, S.bk, st)));
@@ -2447,7 +2483,7 @@ int enqueue_fused_solve(al_engine* e, const StepPlan<TF>& P0, FusedPlan<TF>& F, 
   if (P0.div) {
     ALB_LAUNCH(e, "div_warm1", 1, st, (k_kappa<TF, kDivWarm, false, true><<<G, B, 0, st>>>(c, S)));
     ALB_LAUNCH(e, "div_rho_adv", 1, st,
-               (k_df_rho_adv_init<TF, false, true><<<G, B, 0, st>>>(c, S)));
+               (k_df_rho_adv_init<TF, false, true><<<G, B, 0, st>>>(c, S, none, 0)));
     ALB_TRY(solve(0, [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) -> int {
       ALB_LAUNCH(e, "div_iter", 1, s, (k_kappa<TF, kDivIter, false, true><<<G, B, 0, s>>>(c, S)));
       ALB_LAUNCH(e, "div_residual", 1, s,
@@ -2464,7 +2500,7 @@ int enqueue_fused_solve(al_engine* e, const StepPlan<TF>& P0, FusedPlan<TF>& F, 
     ALB_LAUNCH(e, "press_warm1", 1, st,
                (k_kappa<TF, kPressWarm, false, true><<<G, B, 0, st>>>(c, S)));
     ALB_LAUNCH(e, "press_rho_adv", 1, st,
-               (k_p_rho_adv_init<TF, false, true><<<G, B, 0, st>>>(c, S)));
+               (k_p_rho_adv_init<TF, false, true><<<G, B, 0, st>>>(c, S, none, 0)));
     ALB_TRY(solve(1, [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) -> int {
       ALB_LAUNCH(e, "press_iter", 1, s,
                  (k_kappa<TF, kPressIter, false, true><<<G, B, 0, s>>>(c, S)));

@@ -86,15 +86,21 @@ __global__ void k_step_init(StepState<TF> S) {
 }
 
 // ------------------------------------------------------------ loop control
+// Start of a solver loop: one thread of the pass before it.
 template <class TF>
-__global__ void k_loop_begin(StepState<TF> S, int density_solve,
-                             cudaGraphConditionalHandle handle, int use_handle) {
-  Ctrl<TF>& C = *S.ctrl;
+__device__ __forceinline__ void loop_begin(Ctrl<TF>& C, int density_solve,
+                                           cudaGraphConditionalHandle handle, int use_handle) {
   C.it = 0;
   C.ticket = 0;
   const uint32_t mx = density_solve ? C.max_den : C.max_div;
   C.keep_going = mx > 0;
   if (use_handle) cudaGraphSetConditional(handle, C.keep_going);
+}
+
+template <class TF>
+__global__ void k_loop_begin(StepState<TF> S, int density_solve,
+                             cudaGraphConditionalHandle handle, int use_handle) {
+  loop_begin(*S.ctrl, density_solve, handle, use_handle);
 }
 
 // Loop decision of solver_df.hpp:131-133 / 296-298 and solver_ii.hpp:181-183.
