@@ -51,14 +51,6 @@ struct NoExtra {
 
 namespace {
 
-// Candidates tested per round of the build's scan (loads issued together;
-// measured on B200 per build at 8,388,608 / 1,048,576 particles: 2.79 / 0.354
-// ms at 8, 2.84 / 0.358 at 4, 2.89 / 0.370 at 2, and 3.18 / 0.381 for a
-// branch per candidate).
-constexpr uint32_t kScan = 8;
-static_assert(32 % kScan == 0 && kScan <= kSortedPad,
-              "scan rounds must tile 32 and stay in the pad");
-
 // Two phases per particle.  Phase 1 walks the 3x3 rows of z-contiguous
 // cells around the particle's cell and appends every candidate closer than
 // h to the list, in ascending sorted index; about 1 in 7 candidates is
@@ -82,7 +74,8 @@ static_assert(32 % kScan == 0 && kScan <= kSortedPad,
 template <class TF, class BK, bool FACTOR, class EX, bool WR = false, bool BT = false>
 __global__ void __launch_bounds__(kMaxBlock)
     k_build_neighbors(Cn<TF> c, GridDims g, const uint32_t* __restrict__ cell_start,
-                      const vec4<TF>* __restrict__ xs, uint32_t n, uint32_t stride, BK bk,
+                      const vec4<TF>* __restrict__ xs, ScanSoa<TF> soa, uint32_t n,
+                      uint32_t stride, BK bk,
                       uint32_t* __restrict__ nbr, uint32_t* __restrict__ ncount,
                       TF* __restrict__ rho, TF* __restrict__ alpha, TF* __restrict__ rho_rec,
                       uint32_t* __restrict__ flags, EX ex, FusedBuild fb) {
@@ -128,30 +121,16 @@ __global__ void __launch_bounds__(kMaxBlock)
         const uint32_t b = cell_start[cell_linear(g, cx, cy, z0)];
         const uint32_t e = cell_start[cell_linear(g, cx, cy, z1) + 1];
         // The row's candidates in chunks of 32: the distance tests set one
-        // bit per accepted candidate (branch-free, kScan candidates per
-        // round; a round may read up to kScan - 1 entries past the row, into
-        // the next row or the buffer's kSortedPad spare entries, and their
-        // bits are masked off), then the set bits are appended to the list
-        // in ascending order.
-        for (uint32_t t0 = b; t0 < e; t0 += 32) {
-          const uint32_t m = min(e - t0, 32u);
-          const vec4<TF>* xt = xs + t0;
-          uint32_t acc = 0;
-          for (uint32_t q = 0; q < m; q += kScan) {
-            vec3<TF> xj[kScan];
-#pragma unroll
-            for (uint32_t u = 0; u < kScan; ++u) xj[u] = xyz(__ldg(xt + q + u));
-            uint32_t bits = 0;
-#pragma unroll
-            for (uint32_t u = 0; u < kScan; ++u)
-              bits |= uint32_t(pdist2(c, xi, xj[u]) < c.h2) << u;
-            acc |= bits << q;
-          }
-          if (m < 32) acc &= (1u << m) - 1u;
-          if (s - t0 < m) acc &= ~(1u << (s - t0));  // the particle itself
-          for (; acc; acc &= acc - 1) {
+        // bit per accepted candidate (accept_bits), then the set bits are
+        // appended to the list in ascending order.
+        for (uint32_t t0 = b / kScanAlign * kScanAlign; t0 < e; t0 += 32) {
+          uint32_t acc = row_bits<WR>(c, xi, xs, soa, t0, b, e);
+          if (s - t0 < 32u) acc &= ~(0x80000000u >> (s - t0));  // the particle itself
+          while (acc) {
+            const uint32_t k = __clz(acc);
+            acc &= ~(0x80000000u >> k);
             if (cnt < g.cap_nbr) {
-              grp = uint4{grp.y, grp.z, grp.w, t0 + uint32_t(__ffs(acc) - 1)};
+              grp = uint4{grp.y, grp.z, grp.w, t0 + k};
               if (cnt % kNbrGroup == kNbrGroup - 1) list[size_t(cnt / kNbrGroup) * stride] = grp;
             }
             ++cnt;

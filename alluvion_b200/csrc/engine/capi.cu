@@ -388,10 +388,15 @@ int update_neighbors_impl(al_engine* e, const C* cn, const al_consti* cni, const
   ALB_TRY(e->buf("nbr.count", n, &ncount));
   ALB_TRY(e->buf("sorted.rho", n, &rho));
   ALB_CUDA(cudaMemsetAsync(flags, 0, 4 * sizeof(uint32_t), st));
+  ScanSoa<TF> soa;
+  if (sizeof(TF) == 4 && !c.wrap) {
+    soa.ld = scan_soa_ld(n);
+    ALB_TRY(e->buf("sorted.soa", 3 * soa.ld, &soa.p));
+  }
   GridState gs;
-  ALB_TRY(grid_build<TF>(e, c, g, x, n, xs, flags, gs, st));
+  ALB_TRY(grid_build<TF>(e, c, g, x, n, xs, flags, gs, st, nullptr, soa));
   RefBoundaryKernel<TF> bk{boundary_kernel, gs.perm, n, g.nb};
-  ALB_TRY(build_neighbors_density<TF>(c, g, gs, xs, bk, nbr, ncount, rho, nullptr, nullptr, st));
+  ALB_TRY(build_neighbors_density<TF>(c, g, gs, xs, soa, bk, nbr, ncount, rho, nullptr, nullptr, st));
   ALB_TRY(export_neighbors<TF>(c, g, gs, xs, nbr, ncount, rho, neighbors, num_nbr, density, st));
   if (grid_anomaly)
     ALB_CUDA(cudaMemcpyAsync(grid_anomaly, flags, 3 * sizeof(uint32_t), cudaMemcpyDeviceToDevice,

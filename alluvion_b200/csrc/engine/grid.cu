@@ -268,12 +268,13 @@ inline uint32_t order_blocks(uint32_t ncells) {
 
 template <class TF>
 __global__ void k_gather_x(const TF* __restrict__ x, const uint32_t* __restrict__ perm,
-                           uint32_t n, vec4<TF>* __restrict__ xs) {
+                           uint32_t n, vec4<TF>* __restrict__ xs, ScanSoa<TF> soa) {
   uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   uint32_t i = perm[s];
   vec3<TF> p = ld3(x, i);
   xs[s] = vec4<TF>{p.x, p.y, p.z, TF(0)};
+  soa.put(s, p);
 }
 
 inline uint32_t blocks_for(uint32_t n, int block) { return (n + block - 1) / block; }
@@ -347,7 +348,7 @@ int scan_with_flags(al_engine* e, const uint32_t* count, uint32_t* start, uint32
 template <class TF>
 int grid_build(al_engine* e, const Cn<TF>& c, const GridDims& g, const TF* particle_x,
                uint32_t n, vec4<TF>* xs, uint32_t* flags, GridState& gs, cudaStream_t st,
-               uint32_t* zeroed_count) {
+               uint32_t* zeroed_count, const ScanSoa<TF>& soa) {
   gs.n = n;
   gs.ncells = g.ncells;
   gs.flags = flags;
@@ -372,7 +373,7 @@ int grid_build(al_engine* e, const Cn<TF>& c, const GridDims& g, const TF* parti
                                                       gs.perm);
   k_order_cells<<<order_blocks(g.ncells), kOrderThreads, 0, st>>>(gs.cell_start, g.ncells,
                                                                  gs.perm);
-  if (xs) k_gather_x<TF><<<blocks_for(n, kBlock), kBlock, 0, st>>>(particle_x, gs.perm, n, xs);
+  if (xs) k_gather_x<TF><<<blocks_for(n, kBlock), kBlock, 0, st>>>(particle_x, gs.perm, n, xs, soa);
   ALB_CUDA(cudaGetLastError());
   return AL_OK;
 }
@@ -445,9 +446,10 @@ template int grid_build_fused<float>(al_engine*, float, const uint32_t*,
                                      const SortScene<float>*, uint32_t, uint32_t, uint32_t,
                                      GridState&, cudaStream_t);
 template int grid_build<float>(al_engine*, const Cn<float>&, const GridDims&, const float*,
-                               uint32_t, vec4<float>*, uint32_t*, GridState&, cudaStream_t, uint32_t*);
+                               uint32_t, vec4<float>*, uint32_t*, GridState&, cudaStream_t, uint32_t*,
+                               const ScanSoa<float>&);
 template int grid_build<double>(al_engine*, const Cn<double>&, const GridDims&, const double*,
                                 uint32_t, vec4<double>*, uint32_t*, GridState&, cudaStream_t,
-                                uint32_t*);
+                                uint32_t*, const ScanSoa<double>&);
 
 }  // namespace alb

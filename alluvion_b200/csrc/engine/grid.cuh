@@ -13,6 +13,7 @@
 
 #include "common.cuh"
 #include "engine.hpp"
+#include "scan.cuh"
 
 namespace alb {
 
@@ -31,14 +32,14 @@ struct GridState {
 int grid_build_kernels(uint32_t ncells, bool gather = true);
 
 // Hashes, sorts and gathers positions into `xs` (sorted order, w = 0; null:
-// no gather).  particle_x is the caller's [n][3] array.  `flags` must be zeroed
+// no gather) and soa.  particle_x is the caller's [n][3] array.  `flags` must be zeroed
 // by the caller (it is also used by later passes).  `zeroed_count`: the
 // caller's buffer of ncells + 1 zeros to count in (null: the engine's own,
 // cleared here).
 template <class TF>
 int grid_build(al_engine* e, const Cn<TF>& c, const GridDims& g, const TF* particle_x,
                uint32_t n, vec4<TF>* xs, uint32_t* flags, GridState& gs, cudaStream_t st,
-               uint32_t* zeroed_count = nullptr);
+               uint32_t* zeroed_count = nullptr, const ScanSoa<TF>& soa = ScanSoa<TF>{});
 
 // One scene of a fused batch's sort: its positions (the caller's [n][3]),
 // grid, first cell in the batch's concatenated cells (its ncells cells, then

@@ -16,14 +16,9 @@
 
 #include "common.cuh"
 #include "grid.cuh"
+#include "scan.cuh"
 
 namespace alb {
-
-// Spare entries after the n sorted positions that the build reads: its scan
-// loads candidates in rounds of up to 8 and may read past a row's last
-// candidate (the extra bits are masked off), so every sorted-position
-// buffer passed to the build holds n + kSortedPad entries.
-constexpr uint32_t kSortedPad = 8;
 
 // Entries per list group, where entry k of slot s's list lies (row stride
 // `stride` slots), and the words of a list buffer of n slots.
@@ -96,7 +91,7 @@ constexpr size_t kRecStride = 8;
 // density to rho_rec[s * kRecStride].  Raises flags[2] on neighbor overflow.
 template <class TF, class BK>
 int build_neighbors_density(const Cn<TF>& c, const GridDims& g, const GridState& gs,
-                            const vec4<TF>* xs, const BK& bk, uint32_t* nbr, uint32_t* ncount,
+                            const vec4<TF>* xs, const ScanSoa<TF>& soa, const BK& bk, uint32_t* nbr, uint32_t* ncount,
                             TF* rho, TF* alpha, TF* rho_rec, cudaStream_t st);
 
 // Writes reference-layout outputs in original particle order:

@@ -102,10 +102,12 @@ __device__ __forceinline__ uint32_t bits_index(double w) {
 template <class TF>
 __global__ void k_sample_gather(TF mass, const TF* __restrict__ rho, const TF* __restrict__ v,
                                 const uint32_t* __restrict__ perm, uint32_t n,
-                                vec4<TF>* __restrict__ xs, vec4<TF>* __restrict__ vr) {
+                                vec4<TF>* __restrict__ xs, vec4<TF>* __restrict__ vr,
+                                ScanSoa<TF> soa) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const uint32_t j = perm[t];
+  soa.put(t, xyz(xs[t]));
   xs[t].w = index_bits(j, TF(0));
   if (!rho) return;
   const vec3<TF> u = v ? ld3(v, j) : vec3<TF>{0, 0, 0};
@@ -113,8 +115,7 @@ __global__ void k_sample_gather(TF mass, const TF* __restrict__ rho, const TF* _
 }
 
 // Samples [first, first + num) of the sorted order, without pellets.  Phase 1
-// is the neighbor build's scan (k_build_neighbors: branch-free tests in rounds
-// of kScan, one accept bit each) into a list of up to cap + 1 slots, the spare
+// is the neighbor build's scan (row_bits) into a list of up to cap + 1 slots, the spare
 // one for the particle that shares the sample's index; phase 2 sums over the
 // list.  The vorticity sum_j m / rho_j (v_j - v_s) x grad W needs the
 // sample's own velocity v_s, itself a sum over the list.  With the first
@@ -125,16 +126,12 @@ __global__ void k_sample_gather(TF mass, const TF* __restrict__ rho, const TF* _
 // Both scans of the former two passes ran a branch per candidate and read each
 // neighbor's index, density and velocity in the caller's order: 1.53 ms for
 // 1,048,576 samples among 1,000,000 particles (density, velocity, vorticity,
-// both sorts included), 0.63 ms now (B200).
-constexpr uint32_t kScan = 8;
-static_assert(32 % kScan == 0 && kScan <= kSortedPad,
-              "scan rounds must tile 32 and stay in the pad");
-
+// both sorts included), 0.59 ms now (B200).
 template <class TF, bool WR>
 __global__ void __launch_bounds__(kSampleBlock)
     k_sample_list(Cn<TF> c, GridDims g, const uint32_t* __restrict__ cell_start,
-                  const vec4<TF>* __restrict__ xs, const vec4<TF>* __restrict__ vr,
-                  const vec4<TF>* __restrict__ sample_xs,
+                  const vec4<TF>* __restrict__ xs, ScanSoa<TF> soa,
+                  const vec4<TF>* __restrict__ vr, const vec4<TF>* __restrict__ sample_xs,
                   const uint32_t* __restrict__ sample_perm, uint32_t first, uint32_t num,
                   uint32_t* __restrict__ nbr, SampleDev<TF> sd,
                   const RigidDev<TF>* __restrict__ rigid, uint32_t* flags) {
@@ -167,24 +164,13 @@ __global__ void __launch_bounds__(kSampleBlock)
         if (cy < 0 || cy >= int(g.res[1])) continue;
         const uint32_t b = cell_start[cell_linear(g, cx, cy, z0)];
         const uint32_t e = cell_start[cell_linear(g, cx, cy, z1) + 1];
-        for (uint32_t t0 = b; t0 < e; t0 += 32) {
-          const uint32_t m = min(e - t0, 32u);
-          const vec4<TF>* xt = xs + t0;
-          uint32_t acc = 0;
-          for (uint32_t k = 0; k < m; k += kScan) {
-            V3 xj[kScan];
-#pragma unroll
-            for (uint32_t u = 0; u < kScan; ++u) xj[u] = xyz(__ldg(xt + k + u));
-            uint32_t bits = 0;
-#pragma unroll
-            for (uint32_t u = 0; u < kScan; ++u)
-              bits |= uint32_t(pdist2(c, xi, xj[u]) < c.h2) << u;
-            acc |= bits << k;
-          }
-          if (m < 32) acc &= (1u << m) - 1u;
-          for (; acc; acc &= acc - 1) {
+        for (uint32_t t0 = b / kScanAlign * kScanAlign; t0 < e; t0 += 32) {
+          uint32_t acc = row_bits<WR>(c, xi, xs, soa, t0, b, e);
+          while (acc) {
+            const uint32_t k = __clz(acc);
+            acc &= ~(0x80000000u >> k);
             if (cnt <= g.cap_nbr) {
-              grp = uint4{grp.y, grp.z, grp.w, t0 + uint32_t(__ffs(acc) - 1)};
+              grp = uint4{grp.y, grp.z, grp.w, t0 + k};
               if (cnt % kNbrGroup == kNbrGroup - 1) list[size_t(cnt / kNbrGroup) * num] = grp;
             }
             ++cnt;
@@ -650,18 +636,23 @@ int sample_fluid(al_engine* engine, const typename SampleTypes<TF>::cn* cn, cons
     const uint32_t chunk = sample_chunk(req->num_samples, g.cap_nbr);
     if (need_rho) ALB_TRY(engine->buf("sorted.vr", num_particles ? num_particles : 1, &vr));
     ALB_TRY(engine->buf("list", nbr_list_words(chunk, g.cap_nbr + 1), &list));
+    ScanSoa<TF> soa;
+    if (sizeof(TF) == 4 && !cw.wrap) {
+      soa.ld = scan_soa_ld(num_particles);
+      ALB_TRY(engine->buf("sorted.soa", 3 * soa.ld, &soa.p));
+    }
     if (num_particles)
       ALB_LAUNCH(engine, "sample_gather", 1, st,
                  (k_sample_gather<TF><<<blocks_for(num_particles, kSampleBlock), kSampleBlock, 0,
                                         st>>>(c.mass, need_rho ? req->particle_density : nullptr,
                                               req->sample_v ? req->particle_v : nullptr, gs.perm,
-                                              num_particles, xs, vr)));
+                                              num_particles, xs, vr, soa)));
     for (uint32_t k = 0; k < req->num_samples; k += chunk) {
       const uint32_t m = std::min(chunk, req->num_samples - k);
       ALB_LAUNCH(engine, "sample", 1, st,
                  ((cw.wrap ? k_sample_list<TF, true> : k_sample_list<TF, false>)<<<
                      blocks_for(m, kSampleBlock), kSampleBlock, 0, st>>>(
-                     cw, g1, gs.cell_start, xs, vr, sxs, ss.perm, k, m, list, sd, dr, flags)));
+                     cw, g1, gs.cell_start, xs, soa, vr, sxs, ss.perm, k, m, list, sd, dr, flags)));
     }
   } else {
     ALB_LAUNCH(engine, "sample", 1, st,

@@ -371,6 +371,7 @@ __global__ void k_gather_state(StepState<TF> S, const TF* __restrict__ x_ref,
   }
   const vec3<TF> p = ld3(x_ref, i), v = ld3(v_ref, i);
   S.x[s] = vec4<TF>{p.x, p.y, p.z, TF(0)};
+  S.soa.put(s, p);
   RX(S, s) = vec4<TF>{p.x, p.y, p.z, TF(0)};
   RV(S, s) = vec4<TF>{v.x, v.y, v.z, TF(0)};  // rho follows from the build
   S.kappa[s] = k_ref ? k_ref[i] : TF(0);
@@ -1479,11 +1480,11 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
     ALB_LAUNCH(e, "neighbors", 1, st,
                (wr ? k_build_neighbors<TF, SortedBoundaryKernel<TF>, true, WarmDivergence<TF>, true>
                          <<<blocks_for(n, nbb), nbb, 0, st>>>(
-                             c, P.g, gs.cell_start, S.x, n, S.ls, sbk, S.nbr, S.ncount, S.rho,
+                             c, P.g, gs.cell_start, S.x, S.soa, n, S.ls, sbk, S.nbr, S.ncount, S.rho,
                              S.alpha, rho_rec, gs.flags, wd, FusedBuild{})
                    : k_build_neighbors<TF, SortedBoundaryKernel<TF>, true, WarmDivergence<TF>, false>
                          <<<blocks_for(n, nbb), nbb, 0, st>>>(
-                             c, P.g, gs.cell_start, S.x, n, S.ls, sbk, S.nbr, S.ncount, S.rho,
+                             c, P.g, gs.cell_start, S.x, S.soa, n, S.ls, sbk, S.nbr, S.ncount, S.rho,
                              S.alpha, rho_rec, gs.flags, wd, FusedBuild{})));
     if (P.learned) {
       // inference and its application; in a captured step they sit in an IF
@@ -1511,7 +1512,7 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
     }
   } else
     ALB_LAUNCH(e, "neighbors", 1, st,
-               ALB_TRY(build_neighbors_density<TF>(c, P.g, gs, S.x, sbk, S.nbr, S.ncount, S.rho,
+               ALB_TRY(build_neighbors_density<TF>(c, P.g, gs, S.x, S.soa, sbk, S.nbr, S.ncount, S.rho,
                                                    iisph ? nullptr : S.alpha, rho_rec, st)));
   // One solver loop: `begin`, the pass that forms the solve's first source
   // term, also sets the first condition (loop_begin); `body` launches one
@@ -1851,6 +1852,10 @@ int prepare_step(al_engine* e, const StepArgs<TF>& A, StepPlan<TF>& P, uint32_t 
     P.zeroed_count = reinterpret_cast<uint32_t*>(P.zeroed);
     S.ft = reinterpret_cast<double*>(P.zeroed + count_bytes);
     ALB_TRY(e->buf("sorted.x", size_t(n) + kSortedPad, &S.x));
+    if (sizeof(TF) == 4 && !P.c.wrap) {
+      S.soa.ld = scan_soa_ld(n);
+      ALB_TRY(e->buf("sorted.soa", 3 * S.soa.ld, &S.soa.p));
+    }
     ALB_TRY(e->buf("sorted.rec", size_t(n) * 2, &S.rec));
     ALB_TRY(e->buf("sorted.a", n, &S.a));
     ALB_TRY(e->buf("sorted.rho", n, &S.rho));
@@ -2273,6 +2278,10 @@ int fused_prepare(al_engine* e, std::vector<StepPlan<TF>>& plans, FusedPlan<TF>&
   double* ftp = nullptr;
   e->ns = "fused.";
   ALB_TRY(e->buf("sorted.x", size_t(N) + kSortedPad, &A.x));
+  if (sizeof(TF) == 4) {
+    A.soa.ld = scan_soa_ld(N);
+    ALB_TRY(e->buf("sorted.soa", 3 * A.soa.ld, &A.soa.p));
+  }
   ALB_TRY(e->buf("sorted.rec", size_t(N) * 2, &A.rec));
   ALB_TRY(e->buf("sorted.a", N, &A.a));
   ALB_TRY(e->buf("sorted.rho", N, &A.rho));
@@ -2430,13 +2439,13 @@ int enqueue_fused_head(al_engine* e, const StepPlan<TF>& P0, FusedPlan<TF>& F, c
     const WarmDivergence<TF> wd{S, nullptr, nullptr, c.radius * TF(2), c.vol, nullptr};
     ALB_LAUNCH(e, "neighbors", 1, st,
                (k_build_neighbors<TF, SortedBoundaryKernel<TF>, true, WarmDivergence<TF>, false,
-                                  true><<<G, B, 0, st>>>(c, GridDims{}, nullptr, S.x, 0u, F.N,
+                                  true><<<G, B, 0, st>>>(c, GridDims{}, nullptr, S.x, S.soa, 0u, F.N,
                                                          sbk, S.nbr, S.ncount, S.rho, S.alpha,
                                                          rho_rec, nullptr, wd, fb)));
   } else {
     ALB_LAUNCH(e, "neighbors", 1, st,
                (k_build_neighbors<TF, SortedBoundaryKernel<TF>, true, NoExtra<TF>, false, true>
-                    <<<G, B, 0, st>>>(c, GridDims{}, nullptr, S.x, 0u, F.N, sbk, S.nbr, S.ncount,
+                    <<<G, B, 0, st>>>(c, GridDims{}, nullptr, S.x, S.soa, 0u, F.N, sbk, S.nbr, S.ncount,
                                       S.rho, S.alpha, rho_rec, nullptr, NoExtra<TF>{}, fb)));
   }
   ALB_CUDA(cudaGetLastError());

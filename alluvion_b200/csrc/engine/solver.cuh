@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "engine.hpp"
 #include "grid.cuh"
+#include "scan.cuh"
 
 namespace alb {
 
@@ -65,6 +66,7 @@ struct StepState {
   // SPH); the kernels that write it read only x from its neighbors, so the
   // 4-byte store never races with a value another thread uses.
   vec4<TF>* x = nullptr;
+  ScanSoa<TF> soa;          // the positions as the float scan reads them
   // Interleaved particle records of the passes that gather velocities:
   // rec[2s] = {x, unused}, rec[2s + 1] = {v, rho}, one 32-byte sector (float).
   vec4<TF>* rec = nullptr;
