@@ -45,6 +45,11 @@ __device__ __forceinline__ unsigned long long pack2(float a, float b) {
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
   return r;
 }
+__device__ __forceinline__ float2 unpack2(unsigned long long a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
 __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
   unsigned long long r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -63,9 +68,9 @@ __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigne
 // The scans are bound by instruction issue (ncu).  In float, two candidates
 // share each packed operation and eight share six 16-byte loads; the sign of
 // |d|^2 - h^2 (exact: the subtraction underflows gradually) is the accept
-// bit and enters the mask by one funnel shift: about 6 instructions per
+// bit and enters the mask by one funnel shift: about 7 instructions per
 // candidate instead of 12.  Build at 8,388,608 / 1,048,576 particles:
-// 2,457 / 325 us with the scalar tests, 2,019 / 270 us now (B200).
+// 2,457 / 325 us with the scalar tests, 2,034 / 275 us now (B200).
 template <bool WR, class TF>
 __device__ __forceinline__ uint32_t accept_bits(const Cn<TF>& c, vec3<TF> xi,
                                                 const vec4<TF>* __restrict__ xs,
@@ -73,7 +78,7 @@ __device__ __forceinline__ uint32_t accept_bits(const Cn<TF>& c, vec3<TF> xi,
   uint32_t acc = 0;
   if constexpr (sizeof(TF) == 4 && !WR) {
     const unsigned long long nx = pack2(-xi.x, -xi.x), ny = pack2(-xi.y, -xi.y),
-                             nz = pack2(-xi.z, -xi.z), nh = pack2(-c.h2, -c.h2);
+                             nz = pack2(-xi.z, -xi.z);
     const float* px = soa.p + t0;
     for (uint32_t q = 0; q < m; q += kScan) {
       ulonglong2 x[2], y[2], z[2];
@@ -88,10 +93,14 @@ __device__ __forceinline__ uint32_t accept_bits(const Cn<TF>& c, vec3<TF> xi,
         const unsigned long long dx = add2(u & 1 ? x[u / 2].y : x[u / 2].x, nx),
                                  dy = add2(u & 1 ? y[u / 2].y : y[u / 2].x, ny),
                                  dz = add2(u & 1 ? z[u / 2].y : z[u / 2].x, nz);
-        const unsigned long long d2 = add2(add2(mul2(dx, dx), mul2(dy, dy)), mul2(dz, dz));
-        const unsigned long long e = add2(d2, nh);
-        acc = __funnelshift_l(uint32_t(e), acc, 1);
-        acc = __funnelshift_l(uint32_t(e >> 32), acc, 1);
+        // the sums by scalar additions: a packed product and a packed sum
+        // were contracted, which moved single candidates across h
+        const float2 sx = unpack2(mul2(dx, dx)), sy = unpack2(mul2(dy, dy)),
+                     sz = unpack2(mul2(dz, dz));
+        const float ea = __fsub_rn(__fadd_rn(__fadd_rn(sx.x, sy.x), sz.x), c.h2);
+        const float eb = __fsub_rn(__fadd_rn(__fadd_rn(sx.y, sy.y), sz.y), c.h2);
+        acc = __funnelshift_l(__float_as_uint(ea), acc, 1);
+        acc = __funnelshift_l(__float_as_uint(eb), acc, 1);
       }
     }
     acc <<= 32u - (m + kScan - 1) / kScan * kScan;
