@@ -203,6 +203,17 @@ template <class TF>
 __device__ __forceinline__ vec3<TF> group_sum(vec3<TF> v, const Lane& L) {
   return vec3<TF>{group_sum(v.x, L), group_sum(v.y, L), group_sum(v.z, L)};
 }
+// k times that sum, rounded on its own: contracted into what follows it or
+// not as the compiler pleases, a pass's one-scene and batch forms would differ
+// in the last bits.
+template <class TF>
+__device__ __forceinline__ TF scaled_sum(TF k, TF v, const Lane& L) {
+  return mul_rn(k, group_sum(v, L));
+}
+template <class TF>
+__device__ __forceinline__ vec3<TF> scaled_sum(TF k, vec3<TF> v, const Lane& L) {
+  return vec3<TF>{scaled_sum(k, v.x, L), scaled_sum(k, v.y, L), scaled_sum(k, v.z, L)};
+}
 
 // What a pass gathers of each neighbor.  The gathers bound the pair passes:
 // every lane reads its own neighbor, and the L1 data pipe spends about 14
@@ -297,6 +308,22 @@ constexpr int divergence_blocks() {  // least resident kMaxBlock-thread blocks (
   return sizeof(TF) == 8 ? 4 : WR && !BT ? 6 : 0;
 }
 
+// The boundary terms (v_i - v_b) . (grad W V)_b of a particle's velocity
+// divergence.
+template <class TF>
+__device__ __forceinline__ TF boundary_divergence(const StepState<TF>& S, const Lane& L,
+                                                  vec3<TF> vi) {
+  TF acc = 0;
+  for (uint32_t m = S.mask[L.s]; m; m &= m - 1) {
+    const uint32_t b = __ffs(m) - 1;
+    const vec4<TF> bn = S.bx[size_t(b) * S.ls + L.s];
+    const vec4<TF> kg = S.bk[size_t(b) * S.ls + L.s];
+    const vec3<TF> vj = body_velocity(S.rigid[b], xyz(bn));
+    acc += dot(vi - vj, xyz(kg));
+  }
+  return acc;
+}
+
 // Sum over neighbors of V (v_i - v_j) . grad W_ij plus the boundary terms
 // (v_i - v_b) . (grad W V)_b: the shared body of compute_density_change
 // (runner.hpp:3192-3228) and compute_density_adv (runner.hpp:3493-3523).
@@ -311,15 +338,7 @@ __device__ __forceinline__ TF velocity_divergence(const Cn<TF>& c, const StepSta
     acc += c.vol * dot(vi - xyz(r.v), gradW(c, d));
   });
   acc = group_sum(acc, L);
-  if (L.act) {
-    for (uint32_t m = S.mask[L.s]; m; m &= m - 1) {
-      const uint32_t b = __ffs(m) - 1;
-      const vec4<TF> bn = S.bx[size_t(b) * S.ls + L.s];
-      const vec4<TF> kg = S.bk[size_t(b) * S.ls + L.s];
-      const vec3<TF> vj = body_velocity(S.rigid[b], xyz(bn));
-      acc += dot(vi - vj, xyz(kg));
-    }
-  }
+  if (L.act) acc += boundary_divergence(S, L, vi);
   return acc;
 }
 
@@ -504,8 +523,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_kappa(Cn<TF> c, StepState<TF> S) 
   BlockSpan B;
   if (!block_scene<BT>(S, B)) return;
   // a scene of a fused batch whose solve has converged sits out the
-  // remaining iterations of the others
-  if (BT && (MODE == kDivIter || MODE == kPressIter) && !S.ctrl->keep_going) return;
+  // remaining iterations of the others, and a divergence solve of at most 0
+  // iterations the one before its loop
+  if ((BT ? MODE == kDivIter || MODE == kPressIter : MODE == kDivIter) && !S.ctrl->keep_going)
+    return;
   const Lane L = pair_lane(S, B);
   const TF dt = S.ctrl->dt;
   TF ki = 0;
@@ -519,15 +540,15 @@ __global__ void __launch_bounds__(kMaxBlock) k_kappa(Cn<TF> c, StepState<TF> S) 
     cnt = S.ncount[L.s];
   }
   for_each_neighbor<4>(S, L, cnt, LoadX<TF>{S.x}, [&](uint32_t, const vec4<TF>& xj) {
-    const TF ksum = ki + xj.w;
-    if (fabs(ksum) > c.eps) {
-      const vec3<TF> gw = gradW(c, pdisp(c, xi, xyz(xj)));
-      if (kDiv) {
-        const vec3<TF> gpj = (-c.vol) * gw;
-        dv -= (dt * ksum) * gpj;
-      } else {
-        dv += (dt * ksum * c.vol) * gw;
-      }
+    // a select, not a branch: the neighbors' loads and sums interleave
+    // (625 -> 548 us per pass at 8,388,608 particles)
+    const TF ksum = ki + xj.w, k = fabs(ksum) > c.eps ? ksum : TF(0);
+    const vec3<TF> gw = gradW(c, pdisp(c, xi, xyz(xj)));
+    if (kDiv) {
+      const vec3<TF> gpj = (-c.vol) * gw;
+      dv -= (dt * k) * gpj;
+    } else {
+      dv += (dt * k * c.vol) * gw;
     }
   });
   dv = group_sum(dv, L);
@@ -544,7 +565,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_kappa(Cn<TF> c, StepState<TF> S) 
       const vec3<TF> a = ki * (-xyz(kg));
       f = c.mass * a;
       dv -= dt * a;
-      tq = cross(xyz(bn) - S.rigid[b].x, f);
+      tq = cross_rn(xyz(bn) - S.rigid[b].x, f);
     }
     block_add_ft(S, B.bid, b, f, tq);
   }
@@ -554,6 +575,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_kappa(Cn<TF> c, StepState<TF> S) 
     const vec4<TF> v = RV(S, L.s);
     RV(S, L.s) = vec4<TF>{v.x + dv.x, v.y + dv.y, v.z + dv.z, v.w};
   }
+}
+
+// One neighbor's viscosity over v_i - v_j (compute_viscosity,
+// runner.hpp:2150-2249), by one division; d_gw = d . grad W.
+template <class TF>
+__device__ __forceinline__ TF viscosity_weight(const Cn<TF>& c, TF m_visc, TF r2, TF d_gw,
+                                               TF rho_j) {
+  return mul_rn(m_visc, d_gw) / mul_rn(rho_j, add_rn(r2, mul_rn(TF(0.01), c.h2)));
 }
 
 // compute_velocity_of_density_change (runner.hpp:3297-3314); also forms
@@ -600,10 +629,55 @@ __global__ void __launch_bounds__(kMaxBlock, (divergence_blocks<TF, WR, BT>()))
     finish_iteration(*S.ctrl, total, B.n, 0, handle, use_handle);
 }
 
+// k_df_residual of the divergence solve's first iteration together with the
+// neighbors' viscosity sums, which need the same gathers (a pass of its own
+// spent 974 us per step on them at 8,388,608 particles: 237 are left there, and
+// this pass takes 902 instead of 822).
+// Most solves end here; k_viscosity sums again after one that does not.  In a
+// solve of at most 0 iterations only the viscosity is formed.
+template <class TF, bool WR = false, bool BT = false>
+__global__ void __launch_bounds__(kMaxBlock, sizeof(TF) == 8 ? 3 : 5)
+    k_df_residual_first(Cn<TF> c, StepState<TF> S, cudaGraphConditionalHandle handle,
+                        int use_handle) {
+  if constexpr (!WR) c.wrap = 0;  // non-periodic: the wrap branches fold away
+  BlockSpan B;
+  if (!block_scene<BT>(S, B)) return;
+  scene_bodies<BT>(S, B);
+  const bool run = S.ctrl->keep_going != 0;
+  const Lane L = pair_lane(S, B);
+  const uint32_t cnt = L.act ? S.ncount[L.s] : 0u;
+  const vec3<TF> xi = L.act ? xyz(RX(S, L.s)) : vec3<TF>{0, 0, 0};
+  const vec3<TF> vi = L.act ? xyz(RV(S, L.s)) : vec3<TF>{0, 0, 0};
+  TF adv = 0;
+  vec3<TF> da{0, 0, 0};
+  for_each_neighbor<2>(S, L, cnt, LoadXV<TF>{S}, [&](uint32_t, const NbrXV<TF>& r) {
+    const vec3<TF> d = pdisp(c, xi, xyz(r.x)), dv = vi - xyz(r.v);  // r.v = {v, rho}
+    const vec3<TF> gw = gradW(c, d);
+    adv += c.vol * dot(dv, gw);
+    da += viscosity_weight(c, c.visc * c.mass, length_sqr(d), dot(d, gw), r.v.w) * dv;
+  });
+  da = group_sum(da, L);
+  if (L.lead()) S.a[L.s] = vec4<TF>{da.x, da.y, da.z, TF(0)};
+  if (!run) return;
+  adv = group_sum(adv, L);
+  if (L.act) adv += boundary_divergence(S, L, vi);
+  adv = fmax(adv, TF(0));
+  if (cnt < 20) adv = 0;
+  double val = 0;
+  if (L.lead()) {
+    S.rho_adv[L.s] = adv;
+    S.x[L.s].w = adv * S.alpha[L.s];
+    val = double(adv);
+  }
+  double total;
+  if (grid_sum_last(val, S.red, &S.ctrl->ticket, &total, B.bid, B.nblk) && threadIdx.x == 0)
+    finish_iteration(*S.ctrl, total, B.n, 0, handle, use_handle);
+}
+
 // clear_acceleration + compute_viscosity (runner.hpp:1974-1980, 2150-2249),
 // divergence_solve_finish (runner.hpp:3412-3420) when `finish_div`, and
-// calculate_cfl_v2 (runner.hpp:2533-2541) reduced to the global max; the
-// last block applies Solver::update_dt (solver.hpp:153-169).
+// calculate_cfl_v2 (runner.hpp:2533-2541) reduced to the global max, from
+// which the next pass takes the time step (step_dt).
 //
 // The float kernel is held at 64 registers (8 resident 128-thread blocks per
 // SM): a fused batch's scene lookups would otherwise take it to 76.
@@ -622,14 +696,20 @@ __global__ void __launch_bounds__(kMaxBlock, sizeof(TF) == 4 ? 4 : 1)
     vi = xyz(RV(S, L.s));
     cnt = S.ncount[L.s];
   }
-  for_each_neighbor<xv_batch<TF, WR>()>(S, L, cnt, LoadXV<TF>{S},
-                                        [&](uint32_t, const NbrXV<TF>& r) {
-    const vec3<TF> d = pdisp(c, xi, xyz(r.x));  // r.v = {v, rho}
-    da += (c.visc * c.mass * dot(d, gradW(c, d)) /
-           (r.v.w * (length_sqr(d) + TF(0.01) * c.h2))) *
-          (vi - xyz(r.v));
-  });
-  da = group_sum(da, L);
+  // the divergence solve's first iteration has summed it already, unless
+  // further ones have changed the velocities since
+  const bool summed = finish_div && S.ctrl->it <= 1;
+  if (summed) {
+    if (L.lead()) da = xyz(S.a[L.s]);
+  } else {
+    for_each_neighbor<xv_batch<TF, WR>()>(S, L, cnt, LoadXV<TF>{S},
+                                          [&](uint32_t, const NbrXV<TF>& r) {
+      const vec3<TF> d = pdisp(c, xi, xyz(r.x));  // r.v = {v, rho}
+      da += viscosity_weight(c, c.visc * c.mass, length_sqr(d), dot(d, gradW(c, d)), r.v.w) *
+            (vi - xyz(r.v));
+    });
+    da = group_sum(da, L);
+  }
   scene_bodies<BT>(S, B);
   const uint32_t m = L.lead() ? S.mask[L.s] : 0u;
   const uint32_t nb = block_bodies(S.nb, m);
@@ -648,8 +728,8 @@ __global__ void __launch_bounds__(kMaxBlock, sizeof(TF) == 4 ? 4 : 1)
         // get_orthogonal_vectors (runner.hpp:119-131)
         vec3<TF> ref{TF(1), TF(0), TF(0)};
         if (fabs(dot(ref, nrm)) > TF(0.999)) ref = vec3<TF>{TF(0), TF(1), TF(0)};
-        vec3<TF> t1 = cross(nrm, ref);
-        vec3<TF> t2 = cross(nrm, t1);
+        vec3<TF> t1 = cross_rn(nrm, ref);
+        vec3<TF> t2 = cross_rn(nrm, t1);
         t1 = rsqrt_(dot(t1, t1)) * t1;
         t2 = rsqrt_(dot(t2, t2)) * t2;
         const TF dist = c.h - sqrt(nl2);
@@ -661,16 +741,17 @@ __global__ void __launch_bounds__(kMaxBlock, sizeof(TF) == 4 ? 4 : 1)
         for (int q = 0; q < 4; ++q) {
           const vec3<TF> xix = xi - pts[q];
           const vec3<TF> vb = body_velocity(rg, pts[q]);
-          acc[q] = (c.bvisc * vol * dot(xix, gradW(c, xix)) /
-                    (length_sqr(xix) + TF(0.01) * c.h2)) *
+          const TF r2 = length_sqr(xix);
+          acc[q] = viscosity_weight(c, c.bvisc * vol, r2, radial_grad_rn(c, r2), TF(1)) *
                    (vi - vb);
         }
         da += acc[0] + acc[1] + acc[2] + acc[3];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const vec3<TF> fq = (-c.mass) * acc[q];
+          const vec3<TF> fq{mul_rn(-c.mass, acc[q].x), mul_rn(-c.mass, acc[q].y),
+                            mul_rn(-c.mass, acc[q].z)};
           fsum += fq;
-          tsum += cross(pts[q] - rg.x, fq);
+          tsum += cross_rn(pts[q] - rg.x, fq);
         }
       }
     }
@@ -688,7 +769,6 @@ __global__ void __launch_bounds__(kMaxBlock, sizeof(TF) == 4 ? 4 : 1)
   }
   // block max, then one ordered-bits atomicMax per block
   __shared__ TF wmax[kMaxBlock / 32];
-  __shared__ bool last;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v2 = fmax(v2, __shfl_xor_sync(0xffffffffu, v2, o));
   if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = v2;
@@ -701,23 +781,24 @@ __global__ void __launch_bounds__(kMaxBlock, sizeof(TF) == 4 ? 4 : 1)
       bits = __float_as_uint(bm);
     else
       bits = (unsigned long long)__double_as_longlong(bm);
-    atomicMax(&S.ctrl->vmax_bits, bits);
-    __threadfence();
-    last = atomicAdd(&S.ctrl->ticket, 1u) == B.nblk - 1;
+    // tens of thousands of blocks queue up at one address: only those that
+    // raise the maximum they see write
+    if (bits > __ldcg(&S.ctrl->vmax_bits)) atomicMax(&S.ctrl->vmax_bits, bits);
   }
-  __syncthreads();
-  if (last && threadIdx.x == 0) {
-    Ctrl<TF>& C = *S.ctrl;
-    __threadfence();
-    const unsigned long long bits = atomicAdd(&C.vmax_bits, 0ull);
-    TF pmax;
-    if constexpr (sizeof(TF) == 4)
-      pmax = __uint_as_float(uint32_t(bits));
-    else
-      pmax = __longlong_as_double((long long)bits);
-    apply_update_dt(C, pmax);
-    C.ticket = 0;
-  }
+}
+
+// Solver::update_dt (solver.hpp:153-169) at the head of the pass after
+// k_viscosity: every thread forms the new time step from the maximum, and one
+// (`write`) records it; the pass reads no control field that it writes.
+template <class TF>
+__device__ __forceinline__ TF step_dt(Ctrl<TF>& C, bool write) {
+  TF pmax;
+  if constexpr (sizeof(TF) == 4)
+    pmax = __uint_as_float(uint32_t(C.vmax_bits));
+  else
+    pmax = __longlong_as_double((long long)C.vmax_bits);
+  if (write) apply_update_dt(C, pmax);
+  return updated_dt(C, pmax);
 }
 
 // integrate_non_pressure_acceleration (runner.hpp:3422-3428).
@@ -726,7 +807,7 @@ __global__ void k_integrate_np(StepState<TF> S) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   BlockSpan B;
   if (!block_scene<BT>(S, B) || s >= B.end) return;
-  const TF dt = S.ctrl->dt;
+  const TF dt = step_dt(*S.ctrl, B.bid == 0 && threadIdx.x == 0);
   const vec4<TF> a = S.a[s];
   const vec4<TF> v = RV(S, s);
   RV(S, s) = vec4<TF>{v.x + dt * a.x, v.y + dt * a.y, v.z + dt * a.z, v.w};
@@ -870,7 +951,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_ii_predict0(Cn<TF> c, StepState<T
   });
   dii = group_sum(dii, L);
   if (!L.lead()) return;
-  const TF dt = S.ctrl->dt;
+  const TF dt = step_dt(*S.ctrl, blockIdx.x == 0 && threadIdx.x == 0);
   const vec4<TF> a = S.a[L.s];
   const vec4<TF> v = RV(S, L.s);
   RV(S, L.s) = vec4<TF>{v.x + dt * a.x, v.y + dt * a.y, v.z + dt * a.z, v.w};
@@ -910,11 +991,11 @@ __global__ void __launch_bounds__(kMaxBlock)
                                         [&](uint32_t, const NbrXV<TF>& r) {
     const vec3<TF> gw = gradW(c, pdisp(c, xi, xyz(r.x)));
     const vec3<TF> dji = (dpi * c.rho0) * gw;
-    adv += dt * c.vol * dot(vi - xyz(r.v), gw);
-    aii += c.vol * dot(dii - dji, gw);
+    adv += dot(vi - xyz(r.v), gw);
+    aii += dot(dii - dji, gw);
   });
-  adv = group_sum(adv, L);
-  aii = group_sum(aii, L);
+  adv = scaled_sum(dt * c.vol, adv, L);
+  aii = scaled_sum(c.vol, aii, L);
   if (!L.lead()) return;
   adv += rho / c.rho0;
   for (uint32_t m = S.mask[L.s]; m; m &= m - 1) {
@@ -951,9 +1032,9 @@ __global__ void __launch_bounds__(kMaxBlock) k_ii_iter0(Cn<TF> c, StepState<TF> 
   // (k_ii_predict0) and the pressure afterwards (k_ii_iter1), over rho^2
   vec3<TF> acc{0, 0, 0};
   for_each_neighbor<4>(S, L, cnt, LoadX<TF>{S.x}, [&](uint32_t, const vec4<TF>& xj) {
-    acc -= (c.vol * xj.w) * gradW(c, pdisp(c, xi, xyz(xj)));
+    acc -= xj.w * gradW(c, pdisp(c, xi, xyz(xj)));
   });
-  acc = group_sum(acc, L);
+  acc = scaled_sum(c.vol, acc, L);
   if (!L.lead()) return;
   const TF lp = first ? S.kappa_v[L.s] : S.kappa[L.s];
   if (!first) S.kappa_v[L.s] = lp;
@@ -989,9 +1070,9 @@ __global__ void __launch_bounds__(kMaxBlock)
   };
   for_each_neighbor<4>(S, L, cnt, load, [&](uint32_t, const NbrXV<TF>& r) {
     const vec3<TF> gw = gradW(c, pdisp(c, xi, xyz(r.x)));
-    sum += c.vol * dot(dij_pj - xyz(r.v) + dpi_pi * gw, gw);
+    sum += dot(dij_pj - xyz(r.v) + dpi_pi * gw, gw);
   });
-  sum = group_sum(sum, L);
+  sum = scaled_sum(c.vol, sum, L);
   double val = 0;
   if (L.lead()) {
     for (uint32_t m = S.mask[L.s]; m; m &= m - 1) {
@@ -1043,9 +1124,9 @@ __global__ void __launch_bounds__(kMaxBlock)
       const TF rj = __ldg(S.rho + t);
       dpj = __ldg(S.kappa + t) / (rj * rj);
     }
-    ai -= (c.mass * (dpi + dpj)) * gradW(c, pdisp(c, xi, xyz(xj)));
+    ai -= (dpi + dpj) * gradW(c, pdisp(c, xi, xyz(xj)));
   });
-  ai = group_sum(ai, L);
+  ai = scaled_sum(c.mass, ai, L);
   const uint32_t m = L.lead() ? S.mask[L.s] : 0u;
   const uint32_t nb = block_bodies(S.nb, m);
   for (uint32_t b = 0; b < nb; ++b) {
@@ -1057,7 +1138,7 @@ __global__ void __launch_bounds__(kMaxBlock)
       const vec3<TF> a = (c.rho0 * dpi) * xyz(S.bk[size_t(b) * S.ls + L.s]);
       f = c.mass * a;
       ai -= a;
-      tq = cross(xyz(bn) - S.rigid[b].x, f);
+      tq = cross_rn(xyz(bn) - S.rigid[b].x, f);
     }
     block_add_ft(S, b, f, tq);
   }
@@ -1083,7 +1164,7 @@ template <class TF>
 __global__ void __launch_bounds__(kMaxBlock) k_i_advect(StepState<TF> S) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= S.n) return;
-  const TF dt = S.ctrl->dt;
+  const TF dt = step_dt(*S.ctrl, s == 0);
   const vec4<TF> a = S.a[s];
   const vec4<TF> v = RV(S, s);
   RV(S, s) = vec4<TF>{v.x + dt * a.x, v.y + dt * a.y, v.z + dt * a.z, v.w};
@@ -1120,11 +1201,11 @@ __global__ void __launch_bounds__(kMaxBlock)
     const vec3<TF> d = pdisp(c, xi, xyz(r.x));  // r.v = {v, rho}
     const vec3<TF> gw = gradW(c, d);
     const TF rj = r.v.w;
-    adv += dt * c.vol * dot(vi - xyz(r.v), gw);
-    diag += c.vol * (rho + rj) * dot(d, gw) / (rho * rj * (length_sqr(d) + eps));
+    adv += dot(vi - xyz(r.v), gw);
+    diag += (rho + rj) * dot(d, gw) / (rho * rj * (length_sqr(d) + eps));
   });
-  adv = group_sum(adv, L);
-  diag = group_sum(diag, L);
+  adv = scaled_sum(dt * c.vol, adv, L);
+  diag = scaled_sum(c.vol, diag, L);
   if (!L.lead()) return;
   adv += rho / c.rho0;
   for (uint32_t m = S.mask[L.s]; m; m &= m - 1) {
@@ -1172,9 +1253,10 @@ __global__ void __launch_bounds__(kMaxBlock)
   auto load = [&](uint32_t t) { return NbrXS<TF>{__ldg(xl + t), __ldg(S.irho + t)}; };
   for_each_neighbor<4>(S, L, cnt, load, [&](uint32_t, const NbrXS<TF>& r) {
     const vec3<TF> d = pdisp(c, xi, xyz(r.x));  // (rho_i + rho_j) / (rho_i rho_j) = 1/rho_i + 1/rho_j
-    off -= c.vol * (irho + r.s) * dot(d, gradW(c, d)) / (length_sqr(d) + eps) * r.x.w;
+    const TF r2 = length_sqr(d);
+    off -= (irho + r.s) * dot(d, gradW(c, d)) / (r2 + eps) * r.x.w;
   });
-  off = group_sum(off, L);
+  off = scaled_sum(c.vol, off, L);
   double val = 0;
   if (L.lead()) {
     off *= c.rho0;
@@ -1517,7 +1599,8 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
   // One solver loop: `begin`, the pass that forms the solve's first source
   // term, also sets the first condition (loop_begin); `body` launches one
   // iteration on the given stream.
-  auto solve = [&](uint32_t max_iter, auto&& begin, auto&& body) -> int {
+  // `begin` may hold the first iteration itself (`peeled`).
+  auto solve = [&](uint32_t max_iter, bool peeled, auto&& begin, auto&& body) -> int {
     if (capture) {
       ++*loops;
       return capture_while(
@@ -1530,6 +1613,7 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
     }
     begin(cudaGraphConditionalHandle(0), 0);
     bool go = max_iter > 0;
+    if (go && peeled) ALB_TRY(read_keep_going(S, P.io.hflag, st, &go));
     while (go) {
       ALB_TRY(body(st, cudaGraphConditionalHandle(0), 0));
       ALB_TRY(read_keep_going(S, P.io.hflag, st, &go));
@@ -1544,13 +1628,21 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
         ALB_LAUNCH(e, "div_warm1", 1, st,
                    (wr ? k_kappa<TF, kDivWarm, true><<<pg_, pb_, 0, st>>>(c, Sg_) : k_kappa<TF, kDivWarm, false><<<pg_, pb_, 0, st>>>(c, Sg_)));
       }
-      ALB_TRY(solve(P.io.hc->max_div,
+      ALB_TRY(solve(P.io.hc->max_div, true,
                     [&](cudaGraphConditionalHandle h, int use) {
                       uint32_t pg_, pb_;
                       const StepState<TF> Sg_ = pair_shape("div_rho_adv", pg_, pb_);
                       ALB_LAUNCH(e, "div_rho_adv", 1, st,
                                  (wr ? k_df_rho_adv_init<TF, true><<<pg_, pb_, 0, st>>>(c, Sg_, h, use)
                                      : k_df_rho_adv_init<TF, false><<<pg_, pb_, 0, st>>>(c, Sg_, h, use)));
+                      const StepState<TF> Si_ = pair_shape("div_iter", pg_, pb_);
+                      ALB_LAUNCH(e, "div_iter", 1, st,
+                                 (wr ? k_kappa<TF, kDivIter, true><<<pg_, pb_, 0, st>>>(c, Si_)
+                                     : k_kappa<TF, kDivIter, false><<<pg_, pb_, 0, st>>>(c, Si_)));
+                      const StepState<TF> Sr_ = pair_shape("div_residual", pg_, pb_);
+                      ALB_LAUNCH(e, "div_residual", 1, st,
+                                 (wr ? k_df_residual_first<TF, true><<<pg_, pb_, 0, st>>>(c, Sr_, h, use)
+                                     : k_df_residual_first<TF, false><<<pg_, pb_, 0, st>>>(c, Sr_, h, use)));
                     },
                     [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) -> int {
                       {
@@ -1589,7 +1681,7 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
           ALB_LAUNCH(e, "press_warm1", 1, st,
                      (wr ? k_kappa<TF, kPressWarm, true><<<pg_, pb_, 0, st>>>(c, Sg_) : k_kappa<TF, kPressWarm, false><<<pg_, pb_, 0, st>>>(c, Sg_)));
         }
-        ALB_TRY(solve(P.io.hc->max_den,
+        ALB_TRY(solve(P.io.hc->max_den, false,
                       [&](cudaGraphConditionalHandle h, int use) {
                         uint32_t pg_, pb_;
                         const StepState<TF> Sg_ = pair_shape("press_rho_adv", pg_, pb_);
@@ -1623,7 +1715,7 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
                      f->particle_kappa_v, f->particle_density_adv, P.warm_floor)));
     } else if (P.isph) {
       ALB_LAUNCH(e, "i_advect", 1, st, k_i_advect<TF><<<blocks, kBlock, 0, st>>>(S));
-      ALB_TRY(solve(P.io.hc->max_den,
+      ALB_TRY(solve(P.io.hc->max_den, false,
                     [&](cudaGraphConditionalHandle h, int use) {
                       uint32_t pg_, pb_;
                       const StepState<TF> Sg_ = pair_shape("i_diag", pg_, pb_);
@@ -1658,7 +1750,7 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
         const StepState<TF> Sg_ = pair_shape("ii_predict0", pg_, pb_);
         ALB_LAUNCH(e, "ii_predict0", 1, st, (wr ? k_ii_predict0<TF, true><<<pg_, pb_, 0, st>>>(c, Sg_) : k_ii_predict0<TF, false><<<pg_, pb_, 0, st>>>(c, Sg_)));
       }
-      ALB_TRY(solve(P.io.hc->max_den,
+      ALB_TRY(solve(P.io.hc->max_den, false,
                     [&](cudaGraphConditionalHandle h, int use) {
                       uint32_t pg_, pb_;
                       const StepState<TF> Sg_ = pair_shape("ii_predict1", pg_, pb_);
@@ -1713,6 +1805,12 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
 template <class TF>
 uint32_t iteration_launches(const StepPlan<TF>& P) {
   return P.isph ? 1u : 2u;
+}
+
+// Divergence iterations a step's loop runs: all but the first, which goes
+// before it.
+inline uint32_t loop_divergence(const al_step_report& r) {
+  return r.num_divergence_solve ? r.num_divergence_solve - 1 : 0u;
 }
 
 // Captures one step into an executable graph.  Sets `*exec` to null (and
@@ -2041,7 +2139,7 @@ int run_step(al_engine* e, int method, const typename FluidT<TF>::cn* cn, const 
   if (graph)
     e->launches += graph->fixed_launches +
                    uint64_t(iteration_launches(P)) *
-                       (uint64_t(r.num_divergence_solve) + r.num_density_solve) +
+                       (uint64_t(loop_divergence(r)) + r.num_density_solve) +
                    (P.learned && P.io.hc->warm_ran ? kWarmIfLaunches : 0u);
   return finish_step<TF>(A, P);
 }
@@ -2459,22 +2557,21 @@ int enqueue_fused_solve(al_engine* e, const StepPlan<TF>& P0, FusedPlan<TF>& F, 
   const Cn<TF>& c = P0.c;
   const StepState<TF>& S = F.S;
   const uint32_t G = F.nblocks, B = kFusedBlock;
-  auto solve = [&](int density_solve, auto&& body) -> int {
+  // `first` launches the first iteration where it is not the loop's (as in
+  // enqueue_step, the divergence solve's)
+  auto solve = [&](int density_solve, auto&& first, auto&& body) -> int {
+    auto begin = [&](cudaGraphConditionalHandle h, int use) -> int {
+      ALB_LAUNCH(e, "loop_begin", 1, st,
+                 (k_fused_loop_begin<TF><<<1, 256, 0, st>>>(S.fused, F.K, density_solve, F.go, h,
+                                                             use)));
+      return first(h, use);
+    };
     if (capture) {
       ++*loops;
       return capture_while(
-          e, st,
-          [&](cudaGraphConditionalHandle h) -> int {
-            ALB_LAUNCH(e, "loop_begin", 1, st,
-                       (k_fused_loop_begin<TF><<<1, 256, 0, st>>>(S.fused, F.K, density_solve,
-                                                                   F.go, h, 1)));
-            return AL_OK;
-          },
-          body);
+          e, st, [&](cudaGraphConditionalHandle h) -> int { return begin(h, 1); }, body);
     }
-    ALB_LAUNCH(e, "loop_begin", 1, st,
-               (k_fused_loop_begin<TF><<<1, 256, 0, st>>>(S.fused, F.K, density_solve, F.go,
-                                                           cudaGraphConditionalHandle(0), 0)));
+    ALB_TRY(begin(cudaGraphConditionalHandle(0), 0));
     for (;;) {
       ALB_CUDA(cudaMemcpyAsync(F.hgo, F.go, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
       ALB_CUDA(cudaStreamSynchronize(st));
@@ -2493,12 +2590,22 @@ int enqueue_fused_solve(al_engine* e, const StepPlan<TF>& P0, FusedPlan<TF>& F, 
     ALB_LAUNCH(e, "div_warm1", 1, st, (k_kappa<TF, kDivWarm, false, true><<<G, B, 0, st>>>(c, S)));
     ALB_LAUNCH(e, "div_rho_adv", 1, st,
                (k_df_rho_adv_init<TF, false, true><<<G, B, 0, st>>>(c, S, none, 0)));
-    ALB_TRY(solve(0, [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) -> int {
-      ALB_LAUNCH(e, "div_iter", 1, s, (k_kappa<TF, kDivIter, false, true><<<G, B, 0, s>>>(c, S)));
-      ALB_LAUNCH(e, "div_residual", 1, s,
-                 (k_df_residual<TF, false, true><<<G, B, 0, s>>>(c, S, none, 0)));
-      return cond(s, h, use);
-    }));
+    ALB_TRY(solve(
+        0,
+        [&](cudaGraphConditionalHandle h, int use) -> int {
+          ALB_LAUNCH(e, "div_iter", 1, st,
+                     (k_kappa<TF, kDivIter, false, true><<<G, B, 0, st>>>(c, S)));
+          ALB_LAUNCH(e, "div_residual", 1, st,
+                     (k_df_residual_first<TF, false, true><<<G, B, 0, st>>>(c, S, none, 0)));
+          return cond(st, h, use);
+        },
+        [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) -> int {
+          ALB_LAUNCH(e, "div_iter", 1, s,
+                     (k_kappa<TF, kDivIter, false, true><<<G, B, 0, s>>>(c, S)));
+          ALB_LAUNCH(e, "div_residual", 1, s,
+                     (k_df_residual<TF, false, true><<<G, B, 0, s>>>(c, S, none, 0)));
+          return cond(s, h, use);
+        }));
   }
   ALB_LAUNCH(e, "viscosity", 1, st,
              (k_viscosity<TF, false, true><<<G, B, 0, st>>>(c, S, P0.div ? 1 : 0)));
@@ -2510,7 +2617,8 @@ int enqueue_fused_solve(al_engine* e, const StepPlan<TF>& P0, FusedPlan<TF>& F, 
                (k_kappa<TF, kPressWarm, false, true><<<G, B, 0, st>>>(c, S)));
     ALB_LAUNCH(e, "press_rho_adv", 1, st,
                (k_p_rho_adv_init<TF, false, true><<<G, B, 0, st>>>(c, S, none, 0)));
-    ALB_TRY(solve(1, [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) -> int {
+    auto none_first = [](cudaGraphConditionalHandle, int) -> int { return AL_OK; };
+    ALB_TRY(solve(1, none_first, [&](cudaStream_t s, cudaGraphConditionalHandle h, int use) -> int {
       ALB_LAUNCH(e, "press_iter", 1, s,
                  (k_kappa<TF, kPressIter, false, true><<<G, B, 0, s>>>(c, S)));
       ALB_LAUNCH(e, "press_residual", 1, s,
@@ -2655,8 +2763,8 @@ int run_batch(al_engine* e, const std::vector<StepArgs<TF>>& args, std::vector<i
   uint32_t max_div = 0, max_den = 0;
   for (uint32_t k = 0; k < K; ++k) {
     const al_step_report& r = plans[k].io.hc->rep;
-    iters += uint64_t(r.num_divergence_solve) + r.num_density_solve;
-    max_div = std::max(max_div, r.num_divergence_solve);
+    iters += uint64_t(loop_divergence(r)) + r.num_density_solve;
+    max_div = std::max(max_div, loop_divergence(r));
     max_den = std::max(max_den, r.num_density_solve);
     status[k] = finish_step<TF>(args[k], plans[k]);
   }

@@ -15,7 +15,8 @@ namespace {
 
 template <class TF>
 __device__ __forceinline__ vec3<TF> body_velocity(const RigidDev<TF>& r, vec3<TF> at) {
-  return cross(r.omega, at - r.x) + r.v;
+  const vec3<TF> w = cross_rn(r.omega, at - r.x);
+  return {add_rn(w.x, r.v.x), add_rn(w.y, r.v.y), add_rn(w.z, r.v.z)};
 }
 
 // Deterministic double sum over `nblk` blocks (block `blk` of them): every
@@ -128,12 +129,17 @@ __device__ __forceinline__ void finish_iteration(Ctrl<TF>& C, double total, uint
 // |v + a dt|^2 (calculate_cfl_v2, runner.hpp:2533-2541) and the pile's in
 // the report.
 template <class TF>
+__device__ __forceinline__ TF updated_dt(const Ctrl<TF>& C, TF pmax) {
+  const TF max_v = sqrt(fmax(pmax, TF(C.rep.pile_max_v2)));
+  return fmax(fmin(C.cfl * C.length_scale / max_v, C.max_dt), C.min_dt);
+}
+template <class TF>
 __device__ __forceinline__ void apply_update_dt(Ctrl<TF>& C, TF pmax) {
   const TF pile = TF(C.rep.pile_max_v2);
   const TF max_v2 = fmax(pmax, pile);
   const TF max_v = sqrt(max_v2);
   const TF cfl_dt = C.cfl * C.length_scale / max_v;
-  const TF ndt = fmax(fmin(cfl_dt, C.max_dt), C.min_dt);
+  const TF ndt = updated_dt(C, pmax);
   C.rep.particle_max_v2 = double(pmax);
   C.rep.max_v2 = double(max_v2);
   C.rep.cfl_dt = double(cfl_dt);
