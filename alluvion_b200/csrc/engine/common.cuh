@@ -115,6 +115,15 @@ __device__ __forceinline__ vec3<TF> cross_rn(vec3<TF> a, vec3<TF> b) {
           sub_rn(mul_rn(a.x, b.y), mul_rn(a.y, b.x))};
 }
 
+template <class TF>
+__device__ __forceinline__ vec3<TF> scale_rn(TF k, vec3<TF> a) {
+  return {mul_rn(k, a.x), mul_rn(k, a.y), mul_rn(k, a.z)};
+}
+template <class TF>
+__device__ __forceinline__ TF dot_rn(vec3<TF> a, vec3<TF> b) {
+  return add_rn(add_rn(mul_rn(a.x, b.x), mul_rn(a.y, b.y)), mul_rn(a.z, b.z));
+}
+
 // |a - b|^2 evaluated as ((dx*dx + dy*dy) + dz*dz) with every operation
 // rounded on its own: the order length_sqr(x_i - x_j) has in the reference
 // (runner.hpp:1893-1895), without contraction into FMAs.

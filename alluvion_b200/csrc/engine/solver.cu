@@ -562,8 +562,8 @@ __global__ void __launch_bounds__(kMaxBlock) k_kappa(Cn<TF> c, StepState<TF> S) 
     if (mine) {
       const vec4<TF> bn = S.bx[size_t(b) * S.ls + L.s];
       const vec4<TF> kg = S.bk[size_t(b) * S.ls + L.s];
-      const vec3<TF> a = ki * (-xyz(kg));
-      f = c.mass * a;
+      const vec3<TF> a = scale_rn(ki, -xyz(kg));
+      f = scale_rn(c.mass, a);
       dv -= dt * a;
       tq = cross_rn(xyz(bn) - S.rigid[b].x, f);
     }
@@ -722,7 +722,7 @@ __global__ void __launch_bounds__(kMaxBlock, sizeof(TF) == 4 ? 4 : 1)
       const vec3<TF> bxj = xyz(bn);
       const RigidDev<TF> rg = S.rigid[b];
       vec3<TF> nrm = bxj - xi;
-      const TF nl2 = length_sqr(nrm);
+      const TF nl2 = dot_rn(nrm, nrm);
       if (nl2 > TF(0)) {
         nrm = rsqrt_(nl2) * nrm;
         // get_orthogonal_vectors (runner.hpp:119-131)
@@ -730,26 +730,24 @@ __global__ void __launch_bounds__(kMaxBlock, sizeof(TF) == 4 ? 4 : 1)
         if (fabs(dot(ref, nrm)) > TF(0.999)) ref = vec3<TF>{TF(0), TF(1), TF(0)};
         vec3<TF> t1 = cross_rn(nrm, ref);
         vec3<TF> t2 = cross_rn(nrm, t1);
-        t1 = rsqrt_(dot(t1, t1)) * t1;
-        t2 = rsqrt_(dot(t2, t2)) * t2;
         const TF dist = c.h - sqrt(nl2);
-        const vec3<TF> pts[4] = {bxj - t1 * dist, bxj + t1 * dist, bxj - t2 * dist,
-                                 bxj + t2 * dist};
+        t1 = scale_rn(dist, scale_rn(rsqrt_(dot_rn(t1, t1)), t1));
+        t2 = scale_rn(dist, scale_rn(rsqrt_(dot_rn(t2, t2)), t2));
+        const vec3<TF> pts[4] = {bxj - t1, bxj + t1, bxj - t2, bxj + t2};
         const TF vol = TF(0.25) * bn.w;
         vec3<TF> acc[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const vec3<TF> xix = xi - pts[q];
           const vec3<TF> vb = body_velocity(rg, pts[q]);
-          const TF r2 = length_sqr(xix);
-          acc[q] = viscosity_weight(c, c.bvisc * vol, r2, radial_grad_rn(c, r2), TF(1)) *
-                   (vi - vb);
+          const TF r2 = dot_rn(xix, xix);
+          acc[q] = scale_rn(
+              viscosity_weight(c, c.bvisc * vol, r2, radial_grad_rn(c, r2), TF(1)), vi - vb);
         }
         da += acc[0] + acc[1] + acc[2] + acc[3];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const vec3<TF> fq{mul_rn(-c.mass, acc[q].x), mul_rn(-c.mass, acc[q].y),
-                            mul_rn(-c.mass, acc[q].z)};
+          const vec3<TF> fq = scale_rn(-c.mass, acc[q]);
           fsum += fq;
           tsum += cross_rn(pts[q] - rg.x, fq);
         }
