@@ -106,19 +106,35 @@ struct LaunchShape {
   uint32_t block, tpp;
 };
 
+// The solvers whose passes of a group add to the rigid slots (block_add_ft).
+constexpr uint32_t kForceDf = 1, kForceIi = 2, kForceI = 4;
+
 // The pass groups whose launch shape the table sets: `pair` groups walk
 // neighbor lists and take threads per particle too.
 struct TunableGroup {
   const char* name;
   bool pair;
+  uint32_t forces = 0;
 };
 constexpr TunableGroup kTunable[] = {
-    {"neighbors", false},    {"div_warm1", true},     {"div_rho_adv", true},
-    {"div_iter", true},      {"div_residual", true},  {"viscosity", true},
-    {"press_warm0", true},   {"press_warm1", true},   {"press_rho_adv", true},
-    {"press_iter", true},    {"press_residual", true}, {"ii_predict0", true},
-    {"ii_predict1", true},   {"ii_iter0", true},      {"ii_iter1", true},
-    {"i_diag", true},        {"i_iter", true},        {"finish", true}};
+    {"neighbors", false},
+    {"div_warm1", true, kForceDf},
+    {"div_rho_adv", true},
+    {"div_iter", true, kForceDf},
+    {"div_residual", true},
+    {"viscosity", true, kForceDf | kForceIi | kForceI},
+    {"press_warm0", true},
+    {"press_warm1", true, kForceDf},
+    {"press_rho_adv", true},
+    {"press_iter", true, kForceDf},
+    {"press_residual", true},
+    {"ii_predict0", true},
+    {"ii_predict1", true},
+    {"ii_iter0", true},
+    {"ii_iter1", true},
+    {"i_diag", true},
+    {"i_iter", true},
+    {"finish", true, kForceIi | kForceI}};
 constexpr uint32_t kNumTunable = sizeof(kTunable) / sizeof(kTunable[0]);
 
 struct Lane {
@@ -1784,13 +1800,13 @@ int enqueue_step(al_engine* e, StepPlan<TF>& P, cudaStream_t st, bool capture, i
     }
   }
   if (nb) {
-    if (S.grid > kRigidChunks)
+    if (S.slots > kRigidChunks)
       ALB_LAUNCH(e, "rigid_finish", 2, st,
-                 (k_rigid_partial<<<dim3(kRigidChunks, nb), 256, 0, st>>>(S.ft, S.grid, nb, P.ftp),
+                 (k_rigid_partial<<<dim3(kRigidChunks, nb), 256, 0, st>>>(S.ft, S.slots, nb, P.ftp),
                   k_rigid_finish<TF><<<nb, 256, 0, st>>>(S, P.ftp, kRigidChunks)));
     else
       ALB_LAUNCH(e, "rigid_finish", 1, st,
-                 k_rigid_finish<TF><<<nb, 256, 0, st>>>(S, S.ft, S.grid));
+                 k_rigid_finish<TF><<<nb, 256, 0, st>>>(S, S.ft, S.slots));
   }
   ALB_CUDA(cudaGetLastError());
   // ---- read back: report, rigid state, anomaly flags
@@ -1923,15 +1939,23 @@ int prepare_step(al_engine* e, const StepArgs<TF>& A, StepPlan<TF>& P, uint32_t 
   P.bucket = n ? uint32_t(31 - __builtin_clz(n)) : 0u;
   P.ctx = A.batch;
   S.tpp = pair_tpp(n);
-  // per-block buffers (rigid partials, reduction partials) hold the largest
-  // grid any pair pass of this scene launches
+  // Reduction partials: one per block of the largest grid any pair pass of this
+  // scene may launch.  Rigid slots: one per block of the passes that add to
+  // them, by the shapes they launch with and not by the default shape, because
+  // the totals' order follows from the slot count (rigid_partial): a scene of
+  // a fused batch has a slot per block too, and the same count gives the same
+  // sums.
+  const uint32_t forces = P.isph ? kForceI : iisph ? kForceIi : kForceDf;
   S.grid = pair_blocks(n, S.tpp);
   for (uint32_t k = 0; alloc && k < kNumTunable; ++k) {
     if (!kTunable[k].pair) continue;
     const LaunchShape sh = P.shape(e, kTunable[k].name, true);
-    S.grid = std::max(S.grid, pair_blocks(n, sh.tpp, sh.block));
+    const uint32_t blocks = pair_blocks(n, sh.tpp, sh.block);
+    S.grid = std::max(S.grid, blocks);
+    if (kTunable[k].forces & forces) S.slots = std::max(S.slots, blocks);
   }
   if (S.grid == 0) S.grid = 1;
+  if (S.slots == 0) S.slots = 1;
   // ---- buffers
   if (alloc) {
     // the device copy of the staging slot
@@ -1943,7 +1967,7 @@ int prepare_step(al_engine* e, const StepArgs<TF>& A, StepPlan<TF>& P, uint32_t 
     S.rigid = reinterpret_cast<RigidDev<TF>*>(stage + SL::rigid);
     P.flags = reinterpret_cast<uint32_t*>(stage + SL::flag + 64);
     const size_t count_bytes = SL::up64((size_t(P.g.ncells) + 1) * sizeof(uint32_t));
-    P.zeroed_bytes = count_bytes + size_t(nb ? S.grid : 0) * nb * 6 * sizeof(double);
+    P.zeroed_bytes = count_bytes + size_t(nb ? S.slots : 0) * nb * 6 * sizeof(double);
     ALB_TRY(e->buf("zeroed", P.zeroed_bytes, &P.zeroed));
     P.zeroed_count = reinterpret_cast<uint32_t*>(P.zeroed);
     S.ft = reinterpret_cast<double*>(P.zeroed + count_bytes);

@@ -54,7 +54,7 @@ struct FusedIo;
 
 template <class TF>
 struct StepState {
-  uint32_t n = 0, nb = 0, cap = 0, grid = 0;
+  uint32_t n = 0, nb = 0, cap = 0, grid = 0, slots = 0;
   uint32_t tpp = 1;  // threads per particle of the pair passes (pair_tpp)
   // Stride of the slot-major arrays (nbr [cap / 4][ls][4], bx / bk [nb][ls]): n for
   // one scene; the arena's particle count for the scenes of a fused batch.
@@ -89,7 +89,7 @@ struct StepState {
   vec4<TF>* bk = nullptr;
   const BodyDev<TF>* bodies = nullptr;
   RigidDev<TF>* rigid = nullptr;
-  double* ft = nullptr;   // [grid][nb][6] rigid force/torque partials
+  double* ft = nullptr;   // [slots][nb][6] rigid force/torque partials
   double* red = nullptr;  // [grid] reduction partials
   Ctrl<TF>* ctrl = nullptr;
   const uint32_t* perm = nullptr;

@@ -269,3 +269,48 @@ def test_batch_of_benchmark_scenes_matches_oracle(engine, fused, shape):
         for b in buckets:
             for name, _ in groups:
                 engine.set_launch_shape(name, b, 1, 0, 0)
+
+
+@pytest.mark.parametrize("lattice", [(16, 12, 16), (28, 24, 28)])
+def test_rigid_totals_sum_in_one_order(engine, lattice):
+    """Forces and torques of the fused and the branch form, three bodies on the
+    fluid, bit for bit over eight steps.  The totals sum one slot per block a
+    pass launches, in two stages above 128 slots: 24 and 147 slots here, where
+    the default shape (8 threads per particle) would have 192 and 1,176."""
+    h = lattice[1] * 0.02
+
+    def mk():
+        out = []
+        for seed in range(3):
+            bodies = [dict(shape=_capi.SHAPE_SPHERE, params=[0.03], sign=1.0, resolution=16,
+                           use_distance_grid=True, mass=0.1,
+                           inertia=scenes.sphere_inertia(0.1, 0.03),
+                           x=(0.06 + 0.07 * k, h + 0.035, 0.05 + 0.08 * (k % 2)),
+                           v=(0.1 * k, -0.5, 0.05), omega=(1.0, 0.0, 2.0 - k))
+                      for k in range(3)]
+            out.append(scenes.dam_break(engine, np.float32, lattice, 0.01, (0.9, 0.8, 0.7),
+                                        bodies, seed=seed, volume_resolution=16))
+        return out
+
+    fused, branch = mk(), mk()
+    sps = [scenes.solver_params()] * 3
+    _uniform_batch_shapes(engine, fused, 128, 1)
+    try:
+        dts_f, dts_b = [2e-4] * 3, [2e-4] * 3
+        pushed = 0
+        for _ in range(8):
+            engine.set_batch_fused(True)
+            dts_f, reps_f, _ = scenes.batch_step(engine, fused, sps, dts_f)
+            engine.set_batch_fused(False)
+            dts_b, reps_b, _ = scenes.batch_step(engine, branch, sps, dts_b)
+            for rf, rb in zip(reps_f, reps_b):
+                for b in range(4):
+                    assert list(rf.force[b]) == list(rb.force[b])
+                    assert list(rf.torque[b]) == list(rb.torque[b])
+                    pushed += b > 0 and any(rf.force[b])
+        assert pushed > 3 * 8  # the bodies do touch the fluid
+        for f, b in zip(fused, branch):
+            _states_equal(f, b)
+    finally:
+        engine.set_batch_fused(True)
+        _uniform_batch_shapes(engine, fused, 0, 0)
