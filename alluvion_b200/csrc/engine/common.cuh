@@ -101,28 +101,8 @@ __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, 
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }
 __device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(a, b); }
-
-// a x b with every operation rounded as written: contracted as each pass's
-// registers allow, a pass's one-scene and batch forms would differ in the last
-// bits.
-template <class TF>
-__device__ __forceinline__ vec3<TF> cross_rn(vec3<TF> a, vec3<TF> b) {
-  return {sub_rn(mul_rn(a.y, b.z), mul_rn(a.z, b.y)), sub_rn(mul_rn(a.z, b.x), mul_rn(a.x, b.z)),
-          sub_rn(mul_rn(a.x, b.y), mul_rn(a.y, b.x))};
-}
-
-template <class TF>
-__device__ __forceinline__ vec3<TF> scale_rn(TF k, vec3<TF> a) {
-  return {mul_rn(k, a.x), mul_rn(k, a.y), mul_rn(k, a.z)};
-}
-template <class TF>
-__device__ __forceinline__ TF dot_rn(vec3<TF> a, vec3<TF> b) {
-  return add_rn(add_rn(mul_rn(a.x, b.x), mul_rn(a.y, b.y)), mul_rn(a.z, b.z));
-}
 
 // |a - b|^2 evaluated as ((dx*dx + dy*dy) + dz*dz) with every operation
 // rounded on its own: the order length_sqr(x_i - x_j) has in the reference
@@ -310,17 +290,6 @@ __device__ __forceinline__ vec3<TF> gradW(const Cn<TF>& c, vec3<TF> d) {
   const TF s = q <= TF(0.5) ? (q * TF(3) - TF(2)) * c.inv_h
                             : (q <= TF(1) ? (TF(1) - q) * (q - TF(1)) * inv_rl : TF(0));
   return (c.l * s) * d;
-}
-
-// d . grad W of a displacement of squared length rl2, every operation rounded
-// as written (see cross_rn).
-template <class TF>
-__device__ __forceinline__ TF radial_grad_rn(const Cn<TF>& c, TF rl2) {
-  const TF inv_rl = rl2 > TF(0) ? rsqrt_(rl2) : TF(0);
-  const TF q = mul_rn(mul_rn(rl2, inv_rl), c.inv_h), conj = sub_rn(TF(1), q);
-  const TF near = mul_rn(fma_rn(q, TF(3), TF(-2)), c.inv_h);
-  const TF far = mul_rn(mul_rn(-conj, conj), inv_rl);
-  return mul_rn(mul_rn(c.l, q <= TF(0.5) ? near : (q <= TF(1) ? far : TF(0))), rl2);
 }
 
 // Cell coordinates floor(x / h) - grid_offset (get_ipos, runner.hpp:1827-1831)

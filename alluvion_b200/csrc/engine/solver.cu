@@ -219,17 +219,6 @@ template <class TF>
 __device__ __forceinline__ vec3<TF> group_sum(vec3<TF> v, const Lane& L) {
   return vec3<TF>{group_sum(v.x, L), group_sum(v.y, L), group_sum(v.z, L)};
 }
-// k times that sum, rounded on its own: contracted into what follows it or
-// not as the compiler pleases, a pass's one-scene and batch forms would differ
-// in the last bits.
-template <class TF>
-__device__ __forceinline__ TF scaled_sum(TF k, TF v, const Lane& L) {
-  return mul_rn(k, group_sum(v, L));
-}
-template <class TF>
-__device__ __forceinline__ vec3<TF> scaled_sum(TF k, vec3<TF> v, const Lane& L) {
-  return vec3<TF>{scaled_sum(k, v.x, L), scaled_sum(k, v.y, L), scaled_sum(k, v.z, L)};
-}
 
 // What a pass gathers of each neighbor.  The gathers bound the pair passes:
 // every lane reads its own neighbor, and the L1 data pipe spends about 14
@@ -578,10 +567,10 @@ __global__ void __launch_bounds__(kMaxBlock) k_kappa(Cn<TF> c, StepState<TF> S) 
     if (mine) {
       const vec4<TF> bn = S.bx[size_t(b) * S.ls + L.s];
       const vec4<TF> kg = S.bk[size_t(b) * S.ls + L.s];
-      const vec3<TF> a = scale_rn(ki, -xyz(kg));
-      f = scale_rn(c.mass, a);
+      const vec3<TF> a = ki * (-xyz(kg));
+      f = c.mass * a;
       dv -= dt * a;
-      tq = cross_rn(xyz(bn) - S.rigid[b].x, f);
+      tq = cross(xyz(bn) - S.rigid[b].x, f);
     }
     block_add_ft(S, B.bid, b, f, tq);
   }
@@ -598,7 +587,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_kappa(Cn<TF> c, StepState<TF> S) 
 template <class TF>
 __device__ __forceinline__ TF viscosity_weight(const Cn<TF>& c, TF m_visc, TF r2, TF d_gw,
                                                TF rho_j) {
-  return mul_rn(m_visc, d_gw) / mul_rn(rho_j, add_rn(r2, mul_rn(TF(0.01), c.h2)));
+  return m_visc * d_gw / (rho_j * (r2 + TF(0.01) * c.h2));
 }
 
 // compute_velocity_of_density_change (runner.hpp:3297-3314); also forms
@@ -738,34 +727,35 @@ __global__ void __launch_bounds__(kMaxBlock, sizeof(TF) == 4 ? 4 : 1)
       const vec3<TF> bxj = xyz(bn);
       const RigidDev<TF> rg = S.rigid[b];
       vec3<TF> nrm = bxj - xi;
-      const TF nl2 = dot_rn(nrm, nrm);
+      const TF nl2 = length_sqr(nrm);
       if (nl2 > TF(0)) {
         nrm = rsqrt_(nl2) * nrm;
         // get_orthogonal_vectors (runner.hpp:119-131)
         vec3<TF> ref{TF(1), TF(0), TF(0)};
         if (fabs(dot(ref, nrm)) > TF(0.999)) ref = vec3<TF>{TF(0), TF(1), TF(0)};
-        vec3<TF> t1 = cross_rn(nrm, ref);
-        vec3<TF> t2 = cross_rn(nrm, t1);
+        vec3<TF> t1 = cross(nrm, ref);
+        vec3<TF> t2 = cross(nrm, t1);
+        t1 = rsqrt_(dot(t1, t1)) * t1;
+        t2 = rsqrt_(dot(t2, t2)) * t2;
         const TF dist = c.h - sqrt(nl2);
-        t1 = scale_rn(dist, scale_rn(rsqrt_(dot_rn(t1, t1)), t1));
-        t2 = scale_rn(dist, scale_rn(rsqrt_(dot_rn(t2, t2)), t2));
-        const vec3<TF> pts[4] = {bxj - t1, bxj + t1, bxj - t2, bxj + t2};
+        const vec3<TF> pts[4] = {bxj - t1 * dist, bxj + t1 * dist, bxj - t2 * dist,
+                                 bxj + t2 * dist};
         const TF vol = TF(0.25) * bn.w;
         vec3<TF> acc[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const vec3<TF> xix = xi - pts[q];
           const vec3<TF> vb = body_velocity(rg, pts[q]);
-          const TF r2 = dot_rn(xix, xix);
-          acc[q] = scale_rn(
-              viscosity_weight(c, c.bvisc * vol, r2, radial_grad_rn(c, r2), TF(1)), vi - vb);
+          acc[q] = (c.bvisc * vol * dot(xix, gradW(c, xix)) /
+                    (length_sqr(xix) + TF(0.01) * c.h2)) *
+                   (vi - vb);
         }
         da += acc[0] + acc[1] + acc[2] + acc[3];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const vec3<TF> fq = scale_rn(-c.mass, acc[q]);
+          const vec3<TF> fq = (-c.mass) * acc[q];
           fsum += fq;
-          tsum += cross_rn(pts[q] - rg.x, fq);
+          tsum += cross(pts[q] - rg.x, fq);
         }
       }
     }
@@ -1008,8 +998,8 @@ __global__ void __launch_bounds__(kMaxBlock)
     adv += dot(vi - xyz(r.v), gw);
     aii += dot(dii - dji, gw);
   });
-  adv = scaled_sum(dt * c.vol, adv, L);
-  aii = scaled_sum(c.vol, aii, L);
+  adv = dt * c.vol * group_sum(adv, L);
+  aii = c.vol * group_sum(aii, L);
   if (!L.lead()) return;
   adv += rho / c.rho0;
   for (uint32_t m = S.mask[L.s]; m; m &= m - 1) {
@@ -1048,7 +1038,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_ii_iter0(Cn<TF> c, StepState<TF> 
   for_each_neighbor<4>(S, L, cnt, LoadX<TF>{S.x}, [&](uint32_t, const vec4<TF>& xj) {
     acc -= xj.w * gradW(c, pdisp(c, xi, xyz(xj)));
   });
-  acc = scaled_sum(c.vol, acc, L);
+  acc = c.vol * group_sum(acc, L);
   if (!L.lead()) return;
   const TF lp = first ? S.kappa_v[L.s] : S.kappa[L.s];
   if (!first) S.kappa_v[L.s] = lp;
@@ -1086,7 +1076,7 @@ __global__ void __launch_bounds__(kMaxBlock)
     const vec3<TF> gw = gradW(c, pdisp(c, xi, xyz(r.x)));
     sum += dot(dij_pj - xyz(r.v) + dpi_pi * gw, gw);
   });
-  sum = scaled_sum(c.vol, sum, L);
+  sum = c.vol * group_sum(sum, L);
   double val = 0;
   if (L.lead()) {
     for (uint32_t m = S.mask[L.s]; m; m &= m - 1) {
@@ -1140,7 +1130,7 @@ __global__ void __launch_bounds__(kMaxBlock)
     }
     ai -= (dpi + dpj) * gradW(c, pdisp(c, xi, xyz(xj)));
   });
-  ai = scaled_sum(c.mass, ai, L);
+  ai = c.mass * group_sum(ai, L);
   const uint32_t m = L.lead() ? S.mask[L.s] : 0u;
   const uint32_t nb = block_bodies(S.nb, m);
   for (uint32_t b = 0; b < nb; ++b) {
@@ -1152,7 +1142,7 @@ __global__ void __launch_bounds__(kMaxBlock)
       const vec3<TF> a = (c.rho0 * dpi) * xyz(S.bk[size_t(b) * S.ls + L.s]);
       f = c.mass * a;
       ai -= a;
-      tq = cross_rn(xyz(bn) - S.rigid[b].x, f);
+      tq = cross(xyz(bn) - S.rigid[b].x, f);
     }
     block_add_ft(S, b, f, tq);
   }
@@ -1218,8 +1208,8 @@ __global__ void __launch_bounds__(kMaxBlock)
     adv += dot(vi - xyz(r.v), gw);
     diag += (rho + rj) * dot(d, gw) / (rho * rj * (length_sqr(d) + eps));
   });
-  adv = scaled_sum(dt * c.vol, adv, L);
-  diag = scaled_sum(c.vol, diag, L);
+  adv = dt * c.vol * group_sum(adv, L);
+  diag = c.vol * group_sum(diag, L);
   if (!L.lead()) return;
   adv += rho / c.rho0;
   for (uint32_t m = S.mask[L.s]; m; m &= m - 1) {
@@ -1270,7 +1260,7 @@ __global__ void __launch_bounds__(kMaxBlock)
     const TF r2 = length_sqr(d);
     off -= (irho + r.s) * dot(d, gradW(c, d)) / (r2 + eps) * r.x.w;
   });
-  off = scaled_sum(c.vol, off, L);
+  off = c.vol * group_sum(off, L);
   double val = 0;
   if (L.lead()) {
     off *= c.rho0;

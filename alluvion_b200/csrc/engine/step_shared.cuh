@@ -15,8 +15,7 @@ namespace {
 
 template <class TF>
 __device__ __forceinline__ vec3<TF> body_velocity(const RigidDev<TF>& r, vec3<TF> at) {
-  const vec3<TF> w = cross_rn(r.omega, at - r.x);
-  return {add_rn(w.x, r.v.x), add_rn(w.y, r.v.y), add_rn(w.z, r.v.z)};
+  return cross(r.omega, at - r.x) + r.v;
 }
 
 // Deterministic double sum over `nblk` blocks (block `blk` of them): every

@@ -314,3 +314,41 @@ def test_rigid_totals_sum_in_one_order(engine, lattice):
     finally:
         engine.set_batch_fused(True)
         _uniform_batch_shapes(engine, fused, 0, 0)
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_fused_batch_of_mixed_divergence_counts(engine, graphs):
+    """Scenes whose divergence solves run no, one and several iterations in one
+    batch: the fused form runs the first iteration before its loop and decides
+    per scene whether the viscosity sums formed there still hold.  Equal to the
+    branch form bit for bit, eagerly and captured."""
+    fused, branch = _scenes(engine), _scenes(engine)
+    sps = [scenes.solver_params(), scenes.solver_params(min_divergence_solve=3),
+           scenes.solver_params(max_divergence_solve=0),
+           scenes.solver_params(min_divergence_solve=2, max_divergence_solve=1),
+           scenes.solver_params(min_divergence_solve=2)]
+    _uniform_batch_shapes(engine, fused, 128, 1)
+    engine.set_graph_mode(graphs)
+    try:
+        dts_f, dts_b = [2e-4] * len(fused), [2e-4] * len(branch)
+        for _ in range(4):
+            engine.set_batch_fused(True)
+            dts_f, reps_f, st_f = scenes.batch_step(engine, fused, sps, dts_f)
+            engine.set_batch_fused(False)
+            dts_b, reps_b, st_b = scenes.batch_step(engine, branch, sps, dts_b)
+            assert st_f == st_b == [0] * len(fused)
+            assert dts_f == dts_b
+            for rf, rb in zip(reps_f, reps_b):
+                for key in ("num_divergence_solve", "num_density_solve", "mean_density_error",
+                            "mean_density_change", "max_v2"):
+                    assert getattr(rf, key) == getattr(rb, key), key
+                for b in range(len(rf.force)):
+                    assert list(rf.force[b]) == list(rb.force[b])
+            its = [r.num_divergence_solve for r in reps_f]
+            assert its[0] >= 1 and its[1] >= 3 and its[2:4] == [0, 1] and its[4] >= 2
+        for f, b in zip(fused, branch):
+            _states_equal(f, b)
+    finally:
+        engine.set_graph_mode(True)
+        engine.set_batch_fused(True)
+        _uniform_batch_shapes(engine, fused, 0, 0)
