@@ -115,18 +115,18 @@ __global__ void k_sample_gather(TF mass, const TF* __restrict__ rho, const TF* _
 }
 
 // Samples [first, first + num) of the sorted order, without pellets.  Phase 1
-// is the neighbor build's scan (row_bits) into a list of up to cap + 1 slots, the spare
-// one for the particle that shares the sample's index; phase 2 sums over the
-// list.  The vorticity sum_j m / rho_j (v_j - v_s) x grad W needs the
-// sample's own velocity v_s, itself a sum over the list.  With the first
-// neighbor's velocity u it is
-//   sum_j m / rho_j (v_j - u) x grad W  +  (u - v_s) x sum_j m / rho_j grad W,
-// so one pass serves both, and the terms are as small as the direct form's.
+// is the neighbor build's scan (row_bits) into a list of up to cap + 1 slots,
+// the spare one for the particle that shares the sample's index; phase 2 sums
+// over the list, and over it once more for the vorticity, which needs the
+// sample's own velocity.  Order and operations are k_sample's: the two give the
+// same bits.
 //
-// Both scans of the former two passes ran a branch per candidate and read each
-// neighbor's index, density and velocity in the caller's order: 1.53 ms for
-// 1,048,576 samples among 1,000,000 particles (density, velocity, vorticity,
-// both sorts included), 0.59 ms now (B200).
+// Its two scans ran a branch per candidate and read each neighbor's index,
+// density and velocity in the caller's order: 1.53 ms for 1,048,576 samples
+// among 1,000,000 particles (density, velocity, vorticity, both sorts included),
+// 0.64 ms now (B200).  One pass for velocity and vorticity, relative to the first
+// neighbor's velocity, took 0.60 ms, but its vorticity was further from 64 bits
+// (2.6e-7 instead of 2.5e-7) and is not used.
 template <class TF, bool WR>
 __global__ void __launch_bounds__(kSampleBlock)
     k_sample_list(Cn<TF> c, GridDims g, const uint32_t* __restrict__ cell_start,
@@ -185,54 +185,49 @@ __global__ void __launch_bounds__(kSampleBlock)
       grp = uint4{grp.y, grp.z, grp.w, grp.w};
     list[size_t(len / kNbrGroup) * num] = grp;
   }
-  // ---- phase 2
+  // ---- phase 2: f(index, position, {v, m / rho}) for every neighbor, in list order
   const bool need_vr = vr != nullptr;
-  const bool vort_out = sd.vort != nullptr;
-  TF dens = 0;
-  TF qs[3] = {0, 0, 0};
-  V3 vel{0, 0, 0}, vort{0, 0, 0}, grad{0, 0, 0}, v0{0, 0, 0};
-  uint32_t used = 0, self = 0;
-  constexpr uint32_t kB = 2;
-  for (uint32_t g0 = 0; g0 < len; g0 += kNbrGroup) {
-    const uint4 q4 = list[size_t(g0 / kNbrGroup) * num];  // this thread's own store
-    const uint32_t t[kNbrGroup] = {q4.x, q4.y, q4.z, q4.w};
+  uint32_t self = 0;
+  auto over_list = [&](auto&& f) {
+    constexpr uint32_t kB = 2;
+    uint32_t used = 0;
+    for (uint32_t g0 = 0; g0 < len; g0 += kNbrGroup) {
+      const uint4 q4 = list[size_t(g0 / kNbrGroup) * num];  // this thread's own store
+      const uint32_t t[kNbrGroup] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
-    for (uint32_t h = 0; h < kNbrGroup; h += kB) {
-      vec4<TF> x4[kB], v4[kB];
+      for (uint32_t h = 0; h < kNbrGroup; h += kB) {
+        vec4<TF> x4[kB], v4[kB];
 #pragma unroll
-      for (uint32_t u = 0; u < kB; ++u) {
-        x4[u] = __ldg(xs + t[h + u]);
-        v4[u] = need_vr ? __ldg(vr + t[h + u]) : vec4<TF>{0, 0, 0, 0};
-      }
-#pragma unroll
-      for (uint32_t u = 0; u < kB; ++u) {
-        if (g0 + h + u >= len) break;
-        const uint32_t j = bits_index(x4[u].w);
-        if (j == s) {  // the reference's p_j != p_i
-          self = 1;
-          continue;
+        for (uint32_t u = 0; u < kB; ++u) {
+          x4[u] = __ldg(xs + t[h + u]);
+          v4[u] = need_vr ? __ldg(vr + t[h + u]) : vec4<TF>{0, 0, 0, 0};
         }
-        if (used >= g.cap_nbr) continue;
-        const V3 d = pdisp(c, xi, xyz(x4[u]));
-        const TF w = W_r2(c, pdist2(c, xi, xyz(x4[u])));
-        dens += c.vol * w;
-        if (need_vr) {
-          const TF mr = v4[u].w, mrw = mr * w;
-          for (uint32_t k = 0; k < sd.qdim; ++k)
-            qs[k] += mrw * __ldg(sd.q + size_t(j) * sd.qdim + k);
-          const V3 vj = xyz(v4[u]);
-          vel += mrw * vj;
-          if (vort_out) {
-            if (used == 0) v0 = vj;
-            const V3 gw = mr * gradW(c, d);
-            vort += cross(vj - v0, gw);
-            grad += gw;
+#pragma unroll
+        for (uint32_t u = 0; u < kB; ++u) {
+          if (g0 + h + u >= len) break;
+          const uint32_t j = bits_index(x4[u].w);
+          if (j == s) {  // the reference's p_j != p_i
+            self = 1;
+            continue;
           }
+          if (used++ < g.cap_nbr) f(j, xyz(x4[u]), v4[u]);
         }
-        ++used;
       }
     }
-  }
+  };
+  TF dens = 0;
+  TF qs[3] = {0, 0, 0};
+  V3 vel{0, 0, 0};
+  over_list([&](uint32_t j, const V3& xj, const vec4<TF>& vj) {
+    const TF w = W_r2(c, pdist2(c, xi, xj));
+    dens += c.vol * w;
+    if (need_vr) {
+      const TF mrw = vj.w * w;
+      for (uint32_t k = 0; k < sd.qdim; ++k)
+        qs[k] += mrw * __ldg(sd.q + size_t(j) * sd.qdim + k);
+      vel += mrw * xyz(vj);
+    }
+  });
   if (cnt - self > g.cap_nbr) flags[2] = 1u;
   // volume-map body terms (runner.hpp:2116-2118, 4228-4236, 4310-4321)
   TF bw = 0;
@@ -246,8 +241,11 @@ __global__ void __launch_bounds__(kSampleBlock)
   if (sd.quantity)
     for (uint32_t k = 0; k < sd.qdim; ++k) sd.quantity[size_t(s) * sd.qdim + k] = qs[k];
   if (sd.vel) st3(sd.vel, s, vel);
-  if (vort_out) {
-    vort += cross(v0 - vel, grad);
+  if (sd.vort) {
+    V3 vort{0, 0, 0};
+    over_list([&](uint32_t, const V3& xj, const vec4<TF>& vj) {
+      vort += vj.w * cross(xyz(vj) - vel, gradW(c, pdisp(c, xi, xj)));
+    });
     for (uint32_t b = 0; b < g.nb; ++b) {
       const TF* bk = sd.bker + (size_t(b) * sd.num + s) * 4;
       vort += cross(body_velocity(sd, rigid[b], b, s) - vel, V3{bk[0], bk[1], bk[2]});

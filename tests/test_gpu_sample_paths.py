@@ -1,0 +1,98 @@
+"""The two sampling kernels: the list kernel and the list-free one (which also
+serves pellets) give the same bits, for bodies, quantities, both types and
+periodic grids."""
+import numpy as np
+import pytest
+import torch
+
+from alluvion_b200 import _capi, scenes
+
+pytestmark = pytest.mark.gpu
+
+LIST_FREE = 1 << 26  # a neighbor capacity that the list kernel does not serve
+OUTPUTS = dict(density=1, position_density=1, quantity=3, v=3, vorticity=3)
+
+
+def _dev(a, dtype):
+    return torch.from_numpy(np.ascontiguousarray(a, dtype)).cuda()
+
+
+def _sample(engine, cn, cni, x, rho, v, sx, q=None, rigid=None, bnd=None, wrap=0.0,
+            outputs=("density", "v", "vorticity")):
+    """Status and host outputs of one call; arrays are device tensors."""
+    f64 = x.dtype == torch.float64
+    req = (_capi.SampleF64 if f64 else _capi.SampleF32)()
+    p = lambda t: _capi.ptr(t).value
+    out = {k: torch.zeros((len(sx), OUTPUTS[k]), dtype=x.dtype, device="cuda") for k in outputs}
+    req.sample_x, req.num_samples = p(sx), len(sx)
+    req.particle_density, req.particle_v = p(rho), p(v)
+    if q is not None:
+        req.particle_quantity, req.quantity_dim = p(q), q.shape[1]
+    if bnd is not None:
+        req.sample_boundary, req.sample_boundary_kernel = p(bnd[0]), p(bnd[1])
+    if wrap:
+        req.wrap_y, req.wrap_length = 1, wrap
+    for k, t in out.items():
+        setattr(req, "sample_" + k, p(t))
+    fn = getattr(_capi.lib(), "al_sample_fluid_f64" if f64 else "al_sample_fluid_f32")
+    status = fn(engine.handle, _capi.ptr(cn), _capi.ptr(cni), _capi.ptr(x), len(x),
+                _capi.ptr(rigid) if rigid is not None else None, _capi.ptr(req), None)
+    return status, {k: t.cpu().numpy() for k, t in out.items()}
+
+
+def _cloud(dtype, n, extent, seed):
+    rng = np.random.default_rng(seed)
+    x = rng.random((n, 3)) * extent
+    return (_dev(x, dtype), _dev(1000 + 50 * rng.random(n), dtype),
+            _dev(rng.normal(0, 1, (n, 3)), dtype), _dev(rng.normal(0, 1, (n, 3)), dtype))
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("periodic", [False, True])
+def test_list_and_list_free_sums_agree(engine, dtype, periodic):
+    cn = scenes.make_const(dtype, 0.01)
+    h = float(cn.kernel_radius)
+    extent = np.array([5.3, 6.0, 4.7]) * h
+    x, rho, v, q = _cloud(dtype, 2500, extent, 5)
+    sx = _dev(np.random.default_rng(6).random((3001, 3)) * extent, dtype)
+    got = []
+    for cap in (128, LIST_FREE):
+        cni = scenes.make_consti((0, 0, 0), extent, h, 0, max_num_neighbors_per_particle=cap)
+        if periodic:
+            cni.grid_offset[1], cni.grid_res[1] = 0, 6
+        got.append(_sample(engine, cn, cni, x, rho, v, sx, q, wrap=6 * h if periodic else 0.0,
+                           outputs=OUTPUTS))
+    assert got[0][0] == got[1][0] == 0
+    for k in OUTPUTS:
+        assert np.array_equal(got[0][1][k], got[1][1][k]), k
+    assert np.abs(got[0][1]["vorticity"]).max() > 0
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_list_and_list_free_sums_agree_with_bodies(engine, dtype):
+    """A moving, spinning sphere above the block: the body terms of both."""
+    sphere = dict(shape=_capi.SHAPE_SPHERE, params=[0.04], sign=1.0, resolution=16,
+                  use_distance_grid=True, mass=0.0, x=(0.12, 0.255, 0.11), v=(0.3, -0.1, 0.2),
+                  omega=(1.0, 2.0, -0.5))
+    sc = scenes.dam_break(engine, dtype, (10, 10, 10), 0.01, (0.3, 0.3, 0.3), [sphere], seed=3,
+                          volume_resolution=16)
+    sc.step("df", scenes.solver_params(integrate_rigids=0), 2e-4)
+    rng = np.random.default_rng(8)
+    sx = _dev(rng.random((2000, 3)) * 0.3, dtype)
+    q = _dev(rng.normal(0, 1, (sc.n, 3)), dtype)
+    bnd = [torch.zeros(sc.num_boundaries, len(sx), 4, dtype=sx.dtype, device="cuda")
+           for _ in range(2)]
+    fn = getattr(_capi.lib(), "al_compute_particle_boundary_" +
+                 ("f64" if dtype == np.float64 else "f32"))
+    _capi.check(fn(engine.handle, _capi.ptr(sc.cn), sc.num_boundaries, _capi.ptr(sc.bodies),
+                   _capi.ptr(sc.rigid), _capi.ptr(sx), len(sx), _capi.ptr(bnd[0]),
+                   _capi.ptr(bnd[1]), None), "boundary")
+    assert float(bnd[1].abs().max()) > 0
+    got = []
+    for cap in (64, LIST_FREE):
+        sc.cni.max_num_neighbors_per_particle = cap
+        got.append(_sample(engine, sc.cn, sc.cni, sc.x, sc.density, sc.v, sx, q, sc.rigid, bnd,
+                           outputs=OUTPUTS))
+    assert got[0][0] == got[1][0] == 0
+    for k in OUTPUTS:
+        assert np.array_equal(got[0][1][k], got[1][1][k]), k
