@@ -18,10 +18,10 @@
 // grid; threads take samples in cell order (a warp's samples read the same
 // cells), scan the 3x3 rows of z-contiguous cells around their cell in
 // canonical (cell, index) order as the neighbor build does, and sum every
-// requested output over the compact list in one pass (k_sample_list; with
-// pellets, k_sample sums while it scans).  As in the reference, whose neighbor kernel skips the candidate
-// whose index equals the point's own (p_j != p_i, runner.hpp:1895),
-// particle s is left out of sample s's sums.  With wrap_y the rows follow
+// requested output over the compact list (k_sample_list; with pellets or very
+// large neighbor capacities k_sample sums while it scans).  As in the reference,
+// whose neighbor kernel skips the candidate whose index equals the point's own
+// (p_j != p_i, runner.hpp:1895), particle s is left out of sample s's sums.  With wrap_y the rows follow
 // the reference's (dx, dy, dz) offset order, cells and displacements
 // wrapped in y (make_neighbor_list<1>).  More than
 // max_num_neighbors_per_particle neighbors raise the neighbor-overflow
@@ -254,16 +254,24 @@ __global__ void __launch_bounds__(kSampleBlock)
   }
 }
 
-// Samples per launch of k_sample_list: its list scratch stays within 2^26
-// entries (256 MiB) unless one sample's cap is beyond that.
-inline uint32_t sample_chunk(uint32_t num, uint32_t cap) {
-  const uint64_t per = nbr_list_words(1, cap + 1);
-  const uint64_t most = (uint64_t(1) << 26) / per / kSampleBlock * kSampleBlock;
-  return uint32_t(std::min<uint64_t>(num, std::max<uint64_t>(most, kSampleBlock)));
+// Samples per launch of k_sample_list: its list scratch holds at most 2^26
+// entries (256 MiB).  0 where the list-free kernel serves the call: with
+// pellets, and where so many entries per sample leave less than one block per
+// SM to a launch, unless that is all the samples.  Measured (B200, 1,048,576 /
+// 100,000 samples, 64 neighbors): list-free 1,525 / 488 us; launches of 75,776
+// samples 924 / 258 us, of 37,888 (one block per SM) 1,457 / 300, of 18,944
+// 2,671 / 468, of 4,096 11,372 / 1,525.
+inline uint32_t sample_chunk(uint32_t num, uint32_t npel, uint32_t cap, int num_sms) {
+  const uint64_t per = (uint64_t(cap) + 1 + kNbrGroup - 1) / kNbrGroup * kNbrGroup;
+  const uint64_t most = (uint64_t(1) << 26) / per;
+  if (npel || most < std::min<uint64_t>(num, uint64_t(num_sms) * kSampleBlock)) return 0;
+  return uint32_t(num <= most ? num : most / kSampleBlock * kSampleBlock);
 }
 
-// With pellets.  VORT = false: densities, quantity, velocity; VORT = true: vorticity
-// (reads the samples' velocities written by the first pass).
+// List-free form, with pellets and for calls whose lists would be too large
+// (sample_chunk): sums while it scans.  VORT = false: densities, quantity,
+// velocity; VORT = true: vorticity (reads the samples' velocities written by the
+// first pass).
 template <class TF, bool VORT>
 __global__ void __launch_bounds__(kSampleBlock)
     k_sample(Cn<TF> c, GridDims g, const uint32_t* __restrict__ cell_start,
@@ -626,12 +634,12 @@ int sample_fluid(al_engine* engine, const typename SampleTypes<TF>::cn* cn, cons
   const uint32_t blocks = blocks_for(req->num_samples, kSampleBlock);
   GridDims g1 = g;
   if (!body_terms) g1.nb = 0;  // the first pass reads no body arrays
-  if (npel == 0 && g.cap_nbr < (1u << 26)) {
+  if (const uint32_t chunk =
+          sample_chunk(req->num_samples, npel, g.cap_nbr, engine->num_sms)) {
     Cn<TF> cw = c;
     if (req->wrap_y) set_wrap(cw, TF(req->wrap_length));
     vec4<TF>* vr = nullptr;
     uint32_t* list = nullptr;
-    const uint32_t chunk = sample_chunk(req->num_samples, g.cap_nbr);
     if (need_rho) ALB_TRY(engine->buf("sorted.vr", num_particles ? num_particles : 1, &vr));
     ALB_TRY(engine->buf("list", nbr_list_words(chunk, g.cap_nbr + 1), &list));
     ScanSoa<TF> soa;

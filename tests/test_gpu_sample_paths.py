@@ -96,3 +96,49 @@ def test_list_and_list_free_sums_agree_with_bodies(engine, dtype):
     assert got[0][0] == got[1][0] == 0
     for k in OUTPUTS:
         assert np.array_equal(got[0][1][k], got[1][1][k]), k
+
+
+@pytest.mark.parametrize("cap", [1024, 1767, 1771, 1 << 18, 1 << 20])
+@pytest.mark.parametrize("samples", [1, 5000, 65281, 65282])
+def test_list_scratch_stays_within_256_mib(engine, cap, samples):
+    """A call whose lists do not fit 2^26 entries runs in launches of at least one
+    block per SM, or list-free; results equal the list-free kernel's and the
+    device memory a call takes stays below 256 MiB and the sorted copies."""
+    dtype = np.float32
+    cn = scenes.make_const(dtype, 0.01)
+    h = float(cn.kernel_radius)
+    extent = np.array([4.3, 5.0, 4.7]) * h
+    x, rho, v, _ = _cloud(dtype, 1200, extent, 9)
+    sx = _dev(np.random.default_rng(10).random((samples, 3)) * extent, dtype)
+    per = (cap + 1 + 3) // 4 * 4
+    most = (1 << 26) // per
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if samples <= most:
+        launches = 2  # gather, sums
+    elif most >= sms * 256:
+        launches = 1 + -(-samples // (most // 256 * 256))
+    else:
+        launches = 2  # densities and velocities, vorticity
+    cni = scenes.make_consti((0, 0, 0), extent, h, 0, max_num_particles_per_cell=512,
+                             max_num_neighbors_per_particle=LIST_FREE)
+    _, want = _sample(engine, cn, cni, x, rho, v, sx)
+    cni.max_num_neighbors_per_particle = cap
+    own = _capi.Engine(0)
+    try:
+        tiny = _sample(own, cn, scenes.make_consti((0, 0, 0), extent, h, 0, 512, 64), x, rho, v,
+                       sx[:1])  # the context's own allocations come first
+        assert tiny[0] == 0
+        sorts = own.launch_count()
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        status, got = _sample(own, cn, cni, x, rho, v, sx)
+        torch.cuda.synchronize()
+        taken = free - torch.cuda.mem_get_info()[0]
+        count = own.launch_count() - sorts
+    finally:
+        own.close()
+    assert status == 0
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k
+    assert taken <= (256 + 32) << 20
+    assert count == sorts - 2 + launches  # the two sorts and the sums
