@@ -260,11 +260,15 @@ __global__ void __launch_bounds__(kSampleBlock)
 // SM to a launch, unless that is all the samples.  Measured (B200, 1,048,576 /
 // 100,000 samples, 64 neighbors): list-free 1,525 / 488 us; launches of 75,776
 // samples 924 / 258 us, of 37,888 (one block per SM) 1,457 / 300, of 18,944
-// 2,671 / 468, of 4,096 11,372 / 1,525.
-inline uint32_t sample_chunk(uint32_t num, uint32_t npel, uint32_t cap, int num_sms) {
-  const uint64_t per = (uint64_t(cap) + 1 + kNbrGroup - 1) / kNbrGroup * kNbrGroup;
+// 2,671 / 468, of 4,096 11,372 / 1,525.  Also 0 for a periodic grid of less than
+// three cells along y, where a row is walked more than once: the list's one
+// spare slot would not hold every copy of the sample's own particle.
+inline uint32_t sample_chunk(uint32_t num, uint32_t npel, const GridDims& g, bool wrap,
+                             int num_sms) {
+  const uint64_t per = (uint64_t(g.cap_nbr) + 1 + kNbrGroup - 1) / kNbrGroup * kNbrGroup;
   const uint64_t most = (uint64_t(1) << 26) / per;
-  if (npel || most < std::min<uint64_t>(num, uint64_t(num_sms) * kSampleBlock)) return 0;
+  if (npel || (wrap && g.res[1] < 3)) return 0;
+  if (most < std::min<uint64_t>(num, uint64_t(num_sms) * kSampleBlock)) return 0;
   return uint32_t(num <= most ? num : most / kSampleBlock * kSampleBlock);
 }
 
@@ -635,7 +639,7 @@ int sample_fluid(al_engine* engine, const typename SampleTypes<TF>::cn* cn, cons
   GridDims g1 = g;
   if (!body_terms) g1.nb = 0;  // the first pass reads no body arrays
   if (const uint32_t chunk =
-          sample_chunk(req->num_samples, npel, g.cap_nbr, engine->num_sms)) {
+          sample_chunk(req->num_samples, npel, g, req->wrap_y != 0, engine->num_sms)) {
     Cn<TF> cw = c;
     if (req->wrap_y) set_wrap(cw, TF(req->wrap_length));
     vec4<TF>* vr = nullptr;

@@ -142,3 +142,66 @@ def test_list_scratch_stays_within_256_mib(engine, cap, samples):
         assert np.array_equal(got[k], want[k]), k
     assert taken <= (256 + 32) << 20
     assert count == sorts - 2 + launches  # the two sorts and the sums
+
+
+def _reference(x, s, cn, cni, wrap):
+    """Density sums of every sample in canonical order over its first cap
+    neighbors (float32 tests, float64 sums), and the accepted counts."""
+    f = np.float32
+    h, cap = f(cn.kernel_radius), cni.max_num_neighbors_per_particle
+    off, res = list(cni.grid_offset), list(cni.grid_res)
+    cell = np.floor(x / h).astype(np.int64) - off
+    at = np.floor(s / h).astype(np.int64) - off
+    order = np.lexsort((np.arange(len(x)), cell[:, 2], cell[:, 1], cell[:, 0]))
+    hd = float(h)
+    dens, count = np.zeros(len(s)), np.zeros(len(s), int)
+    for i in range(len(s)):
+        near = []
+        for dx in (-1, 0, 1):
+            for dy in (-1, 0, 1):
+                cy = at[i, 1] + dy
+                if wrap:
+                    cy = cy - res[1] if cy >= res[1] else cy + res[1] if cy < 0 else cy
+                m = ((cell[order, 0] == at[i, 0] + dx) & (cell[order, 1] == cy) &
+                     (np.abs(cell[order, 2] - at[i, 2]) <= 1))
+                j = order[m]
+                d = (s[i] - x[j]).astype(f)
+                if wrap:
+                    y = d[:, 1]
+                    half, full = f(wrap) * f(0.5), f(wrap)
+                    d[:, 1] = np.where(y >= half, y - full, np.where(y < -half, y + full, y))
+                d2 = (d * d)[:, 0] + (d * d)[:, 1] + (d * d)[:, 2]
+                ok = (d2 < h * h) & (j != i)
+                near += list(np.sqrt((d[ok].astype(float) ** 2).sum(1)) / hd)
+        count[i] = len(near)
+        q = np.array(near[:cap])
+        w = np.where(q <= 0.5, (6 * q - 6) * q * q + 1, 2 * (1 - q) ** 3)
+        dens[i] = w.sum() * 8 / np.pi / hd ** 3 * float(cn.particle_vol) * float(cn.density0)
+    return dens, count
+
+
+# float32 sums of up to 200 positive terms with a few rounded operations each:
+# (200 + 20) * 2^-24
+SUM_BOUND = 1.4e-5
+
+
+@pytest.mark.parametrize("cells", [1, 2, 3, 4])
+def test_capacity_of_narrow_periodic_grids(engine, cells):
+    """Periodic grids of one or two cells along y walk a row more than once, and
+    meet the sample's own particle as often: capacities of the accepted count,
+    and one less, with samples on the particles."""
+    cn = scenes.make_const(np.float32, 0.01)
+    h = float(np.float32(cn.kernel_radius))
+    extent = np.array([2.0, cells, 2.0]) * h
+    x, rho, v, _ = _cloud(np.float32, 60, extent, cells)
+    xs = x.cpu().numpy()
+    for spare in (0, -1):
+        cni = scenes.make_consti((0, 0, 0), extent, h, 0, max_num_particles_per_cell=512)
+        cni.grid_offset[1], cni.grid_res[1] = 0, cells
+        cni.max_num_neighbors_per_particle = 10000
+        _, count = _reference(xs, xs, cn, cni, cells * h)
+        cni.max_num_neighbors_per_particle = cap = int(count.max()) + spare
+        want, _ = _reference(xs, xs, cn, cni, cells * h)
+        status, got = _sample(engine, cn, cni, x, rho, v, x, wrap=cells * h)
+        assert status == (_capi.AL_ERR_NEIGHBOR_OVERFLOW if spare else 0)
+        np.testing.assert_allclose(got["density"][:, 0], want, rtol=SUM_BOUND)
