@@ -15,11 +15,6 @@ namespace {
 
 inline uint32_t blocks_for(uint32_t n, int block) { return (n + block - 1) / block; }
 
-template <class TF>
-__device__ __forceinline__ vec3<TF> ldx(const vec4<TF>* p, uint32_t i) {
-  return xyz(__ldg(p + i));
-}
-
 // Record halves of particle s (see StepState::rec).
 template <class TF>
 __device__ __forceinline__ vec4<TF>& RX(const StepState<TF>& S, uint32_t s) {
@@ -634,12 +629,16 @@ __global__ void __launch_bounds__(kMaxBlock, (divergence_blocks<TF, WR, BT>()))
     finish_iteration(*S.ctrl, total, B.n, 0, handle, use_handle);
 }
 
-// k_df_residual of the divergence solve's first iteration together with the
-// neighbors' viscosity sums, which need the same gathers (a pass of its own
-// spent 974 us per step on them at 8,388,608 particles: 237 are left there, and
-// this pass takes 902 instead of 822).
-// Most solves end here; k_viscosity sums again after one that does not.  In a
-// solve of at most 0 iterations only the viscosity is formed.
+// k_df_residual of the divergence solve's first iteration, together with the
+// neighbors' viscosity sums where the solve may end with it: they need the same
+// gathers (8,388,608 particles: this pass 932 us instead of 852, k_viscosity 219
+// instead of 933).  A solve of several iterations changes the velocities again
+// and k_viscosity sums after it.  Where its least and greatest counts say so
+// beforehand, this pass leaves the sums out (two iterations: residuals 1,783 ->
+// 1,705 us); where only the tolerance does, they are lost, 80 us of a 13.7 ms
+// step.  Of 6,000 steps of the 32,768- and 1,048,576-particle dam breaks (0.6 s
+// each) two took more than one iteration.  In a solve of at most 0 iterations
+// only the viscosity is formed.
 template <class TF, bool WR = false, bool BT = false>
 __global__ void __launch_bounds__(kMaxBlock, sizeof(TF) == 8 ? 3 : 5)
     k_df_residual_first(Cn<TF> c, StepState<TF> S, cudaGraphConditionalHandle handle,
@@ -654,18 +653,22 @@ __global__ void __launch_bounds__(kMaxBlock, sizeof(TF) == 8 ? 3 : 5)
   const vec3<TF> xi = L.act ? xyz(RX(S, L.s)) : vec3<TF>{0, 0, 0};
   const vec3<TF> vi = L.act ? xyz(RV(S, L.s)) : vec3<TF>{0, 0, 0};
   TF adv = 0;
-  vec3<TF> da{0, 0, 0};
-  for_each_neighbor<2>(S, L, cnt, LoadXV<TF>{S}, [&](uint32_t, const NbrXV<TF>& r) {
-    const vec3<TF> d = pdisp(c, xi, xyz(r.x)), dv = vi - xyz(r.v);  // r.v = {v, rho}
-    const vec3<TF> gw = gradW(c, d);
-    adv += c.vol * dot(dv, gw);
-    da += viscosity_weight(c, c.visc * c.mass, length_sqr(d), dot(d, gw), r.v.w) * dv;
-  });
-  da = group_sum(da, L);
-  if (L.lead()) S.a[L.s] = vec4<TF>{da.x, da.y, da.z, TF(0)};
-  if (!run) return;
-  adv = group_sum(adv, L);
-  if (L.act) adv += boundary_divergence(S, L, vi);
+  if (min(S.ctrl->min_div, S.ctrl->max_div) <= 1) {
+    vec3<TF> da{0, 0, 0};
+    for_each_neighbor<2>(S, L, cnt, LoadXV<TF>{S}, [&](uint32_t, const NbrXV<TF>& r) {
+      const vec3<TF> d = pdisp(c, xi, xyz(r.x)), dv = vi - xyz(r.v);  // r.v = {v, rho}
+      const vec3<TF> gw = gradW(c, d);
+      adv += c.vol * dot(dv, gw);
+      da += viscosity_weight(c, c.visc * c.mass, length_sqr(d), dot(d, gw), r.v.w) * dv;
+    });
+    da = group_sum(da, L);
+    if (L.lead()) S.a[L.s] = vec4<TF>{da.x, da.y, da.z, TF(0)};
+    if (!run) return;
+    adv = group_sum(adv, L);
+    if (L.act) adv += boundary_divergence(S, L, vi);
+  } else {  // at least two iterations
+    adv = velocity_divergence<WR>(c, S, L, xi, vi, cnt);
+  }
   adv = fmax(adv, TF(0));
   if (cnt < 20) adv = 0;
   double val = 0;
