@@ -98,8 +98,8 @@ def test_sort_over_few_and_many_scan_tiles(engine, res):
 
 @pytest.mark.parametrize("samples", [1, 255, 256, 257, 1500])
 def test_samples_in_chunks(engine, samples):
-    """A neighbor capacity so large that the list scratch holds one block of
-    samples per launch gives what one launch gives, bit for bit."""
+    """A neighbor capacity whose lists would not fit the scratch (served by the
+    list-free kernel) gives what lists give, bit for bit."""
     cn = scenes.make_const(np.float32, 0.01)
     h = float(cn.kernel_radius)
     x = scenes.fluid_block((12, 11, 10), (0, 0, 0), 0.01, np.float32, seed=1)
@@ -125,8 +125,6 @@ def test_samples_in_chunks(engine, samples):
         out.append([t.cpu().numpy() for t in (den, vel, vort)])
     for a, b in zip(*out):
         assert np.array_equal(a, b)
-    # a moving frame: velocities shift by a constant, vorticity by its sum's
-    # share of it only (u - v_s weighs the gradient sum)
     assert np.isfinite(out[0][2]).all()
 
 
@@ -155,3 +153,31 @@ def test_loops_of_no_iteration_or_several(engine, dtype, method, sp):
     assert dt == pytest.approx(odt, rel=tol["dt"])
     for key, bound in (("x", "x"), ("v", "v"), ("density", "density")):
         _close(g[key], ostate[key], tol[bound], key)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_boundary_stop_at_zero_cells_changes_nothing(engine, dtype):
+    """A step that exports the dense boundary terms evaluates every pair, one that
+    does not stops at map cells whose nodes are all 0: equal states, and as many
+    active pairs as the dense terms have volumes."""
+    out = []
+    for dense in (False, True):
+        sc = _scene(engine, dtype)
+        nb = sc.num_boundaries
+        terms = [torch.full((nb, sc.n, 4), -1.0, dtype=sc.tdtype, device="cuda")
+                 for _ in range(2)]
+        if dense:
+            bufs = type(sc).fluid(sc, terms)
+            sc.fluid = lambda: bufs
+        dt = 1e-4
+        for _ in range(3):
+            dt, rep = sc.step("df", scenes.solver_params(), dt)
+        out.append((dt, rep.num_active_boundary_pairs, sc.state(),
+                    scenes.rigid_array(sc.dtype, [sc.rigid[b] for b in range(nb)])))
+    (dt0, pairs0, a, rig0), (dt1, pairs1, b, rig1) = out
+    volumes = terms[0][..., 3]
+    assert pairs0 == pairs1 == int((volumes != 0).sum())
+    assert 0 < pairs0 < volumes.numel()  # both kinds occur
+    assert dt0 == dt1 and np.array_equal(rig0, rig1)
+    for key in a:
+        assert np.array_equal(a[key], b[key]), key

@@ -205,3 +205,66 @@ def test_capacity_of_narrow_periodic_grids(engine, cells):
         status, got = _sample(engine, cn, cni, x, rho, v, x, wrap=cells * h)
         assert status == (_capi.AL_ERR_NEIGHBOR_OVERFLOW if spare else 0)
         np.testing.assert_allclose(got["density"][:, 0], want, rtol=SUM_BOUND)
+
+
+@pytest.mark.parametrize("own", [False, True])
+@pytest.mark.parametrize("spare", [-2, -1, 0, 1])
+def test_capacity_edges(engine, own, spare):
+    """Forty particles within h of every sample: capacities from two below the
+    accepted count to one above it, for samples that share an index with one of
+    the forty (own; it is anywhere in the list, the first and the last entry
+    among them) and for samples that do not."""
+    cn = scenes.make_const(np.float32, 0.01)
+    h = float(np.float32(cn.kernel_radius))
+    rng = np.random.default_rng(12)
+    xs = (1.5 * h + 0.25 * h * (2 * rng.random((40, 3)) - 1)).astype(np.float32)
+    ss = (1.5 * h + 0.1 * h * (2 * rng.random((40, 3)) - 1)).astype(np.float32)
+    if not own:  # samples 0..39 elsewhere, the next ones among the particles
+        ss = np.concatenate([np.full((40, 3), 5.5 * h, np.float32), ss])
+    x, sx = _dev(xs, np.float32), _dev(ss, np.float32)
+    rho = torch.full((40,), 1000.0, device="cuda")
+    cni = scenes.make_consti((0, 0, 0), (6 * h,) * 3, h, 0)
+    accepted = 39 if own else 40
+    cni.max_num_neighbors_per_particle = accepted + spare
+    want, count = _reference(xs, ss, cn, cni, 0.0)
+    assert set(count) == ({39} if own else {0, 40})
+    status, got = _sample(engine, cn, cni, x, rho, torch.zeros_like(x), sx,
+                          outputs=("density", "v"))
+    assert status == (_capi.AL_ERR_NEIGHBOR_OVERFLOW if spare < 0 else 0)
+    np.testing.assert_allclose(got["density"][:, 0], want, rtol=SUM_BOUND)
+
+
+@pytest.mark.parametrize("frame", [0.0, 100.0])
+def test_velocity_and_vorticity_in_a_moving_frame(engine, frame):
+    """Float sums against 64-bit ones, at rest and with a large common velocity;
+    the vorticity against the sample's velocity that the call returned.  Bound:
+    one rounding per term and sum and about 20 in the kernel's factors, on the
+    sum of the terms' magnitudes (the gradient's by its maximum over q)."""
+    cn = scenes.make_const(np.float32, 0.01)
+    h = float(np.float32(cn.kernel_radius))
+    extent = np.array([4.3, 5.0, 4.7]) * h
+    x, rho, v, _ = _cloud(np.float32, 1200, extent, 13)
+    v += frame
+    sx = _dev(np.random.default_rng(14).random((400, 3)) * extent, np.float32)
+    cni = scenes.make_consti((0, 0, 0), extent, h, 0, max_num_neighbors_per_particle=128)
+    status, got = _sample(engine, cn, cni, x, rho, v, sx)
+    assert status == 0
+    xs, vs, rs, ps = (t.cpu().numpy().astype(float) for t in (x, v, rho, sx))
+    mass = float(cn.particle_mass)
+    k, l = 8 / np.pi / h ** 3, 48 / np.pi / h ** 4
+    eps = 2.0 ** -23
+    for i in range(len(ps)):
+        d = ps[i] - xs
+        r = np.sqrt((d ** 2).sum(1))
+        near = (r < h) & (np.arange(len(xs)) != i)
+        d, r, mr, vj = d[near], r[near], (mass / rs)[near], vs[near]
+        q = r / h
+        w = k * np.where(q <= 0.5, (6 * q - 6) * q * q + 1, 2 * (1 - q) ** 3)
+        s = l * np.where(q <= 0.5, (3 * q - 2) / h, -(1 - q) ** 2 / r)
+        n = near.sum() + 20
+        want = ((mr * w)[:, None] * vj).sum(0)
+        assert np.abs(got["v"][i] - want).max() <= n * eps * (mr * w @ np.abs(vj)).max()
+        rel = vj - got["v"][i].astype(float)
+        want = (mr[:, None] * np.cross(rel, s[:, None] * d)).sum(0)
+        scale = (mr * np.sqrt((rel ** 2).sum(1))).sum() * l / 3  # |grad W| <= l / 3
+        assert np.abs(got["vorticity"][i] - want).max() <= n * eps * scale
