@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kMaxBlock)
         // The row's candidates in chunks of 32: the distance tests set one
         // bit per accepted candidate (accept_bits), then the set bits are
         // appended to the list in ascending order.
-        for (uint32_t t0 = b / kScanAlign * kScanAlign; t0 < e; t0 += 32) {
+        for (uint32_t t0 = scan_start<TF, WR>(b); t0 < e; t0 += 32) {
           uint32_t acc = row_bits<WR>(c, xi, xs, soa, t0, b, e);
           if (s - t0 < 32u) acc &= ~(0x80000000u >> (s - t0));  // the particle itself
           while (acc) {

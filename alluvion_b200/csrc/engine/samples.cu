@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kSampleBlock)
         if (cy < 0 || cy >= int(g.res[1])) continue;
         const uint32_t b = cell_start[cell_linear(g, cx, cy, z0)];
         const uint32_t e = cell_start[cell_linear(g, cx, cy, z1) + 1];
-        for (uint32_t t0 = b / kScanAlign * kScanAlign; t0 < e; t0 += 32) {
+        for (uint32_t t0 = scan_start<TF, WR>(b); t0 < e; t0 += 32) {
           uint32_t acc = row_bits<WR>(c, xi, xs, soa, t0, b, e);
           while (acc) {
             const uint32_t k = __clz(acc);

@@ -37,8 +37,18 @@ namespace {
 constexpr uint32_t kScan = 8;
 static_assert(32 % kScan == 0 && kScan <= kSortedPad,
               "scan rounds must tile 32 and stay in the pad");
-// Scans start at multiples of kScanAlign slots, for 16-byte loads.
-constexpr uint32_t kScanAlign = 4;
+// Packed scans (float, not periodic) start at multiples of four slots, for their
+// 16-byte loads; the scalar ones at the row's first slot, because the slots
+// before it cost them up to a round of eight per row (1,331,000 particles in
+// double, neighbor update without rows: 829 us aligned, 692 us so).
+template <class TF, bool WR>
+constexpr bool packed_scan() {
+  return sizeof(TF) == 4 && !WR;
+}
+template <class TF, bool WR>
+__device__ __forceinline__ uint32_t scan_start(uint32_t b) {
+  return packed_scan<TF, WR>() ? b / 4 * 4 : b;
+}
 
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {
   unsigned long long r;
@@ -61,8 +71,8 @@ __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigne
   return r;
 }
 
-// Bit 31 - k of the result: candidate t0 + k (k < m <= 32, t0 a multiple of
-// kScanAlign) is closer than h to xi, by the rounded operations of pdist2.
+// Bit 31 - k of the result: candidate t0 + k (k < m <= 32, t0 a multiple of four
+// in packed scans) is closer than h to xi, by the rounded operations of pdist2.
 // The other bits are 0.
 //
 // The scans are bound by instruction issue (ncu).  In float, two candidates
@@ -76,7 +86,7 @@ __device__ __forceinline__ uint32_t accept_bits(const Cn<TF>& c, vec3<TF> xi,
                                                 const vec4<TF>* __restrict__ xs,
                                                 const ScanSoa<TF>& soa, uint32_t t0, uint32_t m) {
   uint32_t acc = 0;
-  if constexpr (sizeof(TF) == 4 && !WR) {
+  if constexpr (packed_scan<TF, WR>()) {
     const unsigned long long nx = pack2(-xi.x, -xi.x), ny = pack2(-xi.y, -xi.y),
                              nz = pack2(-xi.z, -xi.z);
     const float* px = soa.p + t0;
@@ -93,8 +103,12 @@ __device__ __forceinline__ uint32_t accept_bits(const Cn<TF>& c, vec3<TF> xi,
         const unsigned long long dx = add2(u & 1 ? x[u / 2].y : x[u / 2].x, nx),
                                  dy = add2(u & 1 ? y[u / 2].y : y[u / 2].x, ny),
                                  dz = add2(u & 1 ? z[u / 2].y : z[u / 2].x, nz);
-        // the sums by scalar additions: a packed product and a packed sum
-        // were contracted, which moved single candidates across h
+        // The sums by scalar additions: nvcc 12.9 contracts a packed product
+        // and a packed sum although both say .rn, which moved single
+        // candidates across h.  A scalar __fadd_rn is never contracted by its
+        // definition; that it holds for a packed product as well rests on the
+        // exact list tests (test_config2_neighbor_lists_bit_exact and
+        // test_lists_at_group_and_round_edges): run them with a new toolkit.
         const float2 sx = unpack2(mul2(dx, dx)), sy = unpack2(mul2(dy, dy)),
                      sz = unpack2(mul2(dz, dz));
         const float ea = __fsub_rn(__fadd_rn(__fadd_rn(sx.x, sy.x), sz.x), c.h2);
@@ -120,7 +134,7 @@ __device__ __forceinline__ uint32_t accept_bits(const Cn<TF>& c, vec3<TF> xi,
 }
 
 // accept_bits of the part of row [b, e) in the chunk of 32 slots at t0
-// (t0 <= b in the first chunk only); *m = slots of the chunk.
+// (t0 <= b in the first chunk only).
 template <bool WR, class TF>
 __device__ __forceinline__ uint32_t row_bits(const Cn<TF>& c, vec3<TF> xi,
                                              const vec4<TF>* __restrict__ xs,
