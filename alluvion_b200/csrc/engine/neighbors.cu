@@ -12,10 +12,12 @@ inline uint32_t blocks_for(uint32_t n, int block) { return (n + block - 1) / blo
 // Threads per particle of the export: eight 16-byte entries (float) fill a
 // 128-byte line of the particle's row.  One thread per particle stored its
 // entries 1 KB apart from its neighbors' lanes: 455 us for 306,525 particles
-// with 64-entry rows, 240 us with eight (B200, whole update).
+// with 64-entry rows, 240 us with eight (B200, whole update).  Without rows there
+// is one count and one density per particle, and one thread (512,000 particles,
+// eight threads 19.4 us, one 7.1).
 constexpr uint32_t kExportLanes = 8;
 
-template <class TF>
+template <class TF, uint32_t LANES>
 __global__ void k_export_neighbors(Cn<TF> c, uint32_t cap, uint32_t n,
                                    const uint32_t* __restrict__ perm,
                                    const vec4<TF>* __restrict__ xs,
@@ -23,8 +25,8 @@ __global__ void k_export_neighbors(Cn<TF> c, uint32_t cap, uint32_t n,
                                    const uint32_t* __restrict__ ncount,
                                    const TF* __restrict__ rho_sorted, TF* __restrict__ out_nbr,
                                    uint32_t* __restrict__ out_num, TF* __restrict__ out_rho) {
-  const uint32_t s = blockIdx.x * (blockDim.x / kExportLanes) + threadIdx.x / kExportLanes;
-  const uint32_t lane = threadIdx.x % kExportLanes;
+  const uint32_t s = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES;
+  const uint32_t lane = threadIdx.x % LANES;
   if (s >= n) return;
   const uint32_t i = perm[s];
   const uint32_t cnt = ncount[s];
@@ -36,7 +38,7 @@ __global__ void k_export_neighbors(Cn<TF> c, uint32_t cap, uint32_t n,
   const vec3<TF> xi = xyz(xs[s]);
   // the caller's buffer may start anywhere
   const bool aligned = reinterpret_cast<uintptr_t>(out_nbr) % sizeof(vec4<TF>) == 0;
-  for (uint32_t k = lane; k < cnt; k += kExportLanes) {
+  for (uint32_t k = lane; k < cnt; k += LANES) {
     const uint32_t t = nbr[nbr_index(k, s, n)];
     const uint32_t j = perm[t];
     const vec3<TF> xj = xyz(xs[t]);
@@ -95,8 +97,10 @@ int export_neighbors(const Cn<TF>& c, const GridDims& g, const GridState& gs,
                      TF* particle_neighbors, uint32_t* particle_num_neighbors,
                      TF* particle_density, cudaStream_t st) {
   if (gs.n == 0) return AL_OK;
-  const uint32_t blocks = (gs.n + kBlock / kExportLanes - 1) / (kBlock / kExportLanes);
-  k_export_neighbors<TF><<<blocks, kBlock, 0, st>>>(
+  const uint32_t lanes = particle_neighbors ? kExportLanes : 1;
+  const auto kernel =
+      particle_neighbors ? k_export_neighbors<TF, kExportLanes> : k_export_neighbors<TF, 1>;
+  kernel<<<blocks_for(gs.n, int(kBlock / lanes)), kBlock, 0, st>>>(
       c, g.cap_nbr, gs.n, gs.perm, xs, nbr, ncount, rho_sorted, particle_neighbors,
       particle_num_neighbors, particle_density);
   ALB_CUDA(cudaGetLastError());
