@@ -59,15 +59,17 @@ __device__ __forceinline__ void sample_body(const Cn<TF>& c, const BodyDev<TF>& 
   int ip[3];
   vec3<TF> xi;
   const bool inside = resolve(b, local, ip, xi);
-  bool any = false;
-  if (inside) {
+  if (!dense) {
+    bool any = false;
+    if (inside) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      any |= __ldg(b.vol + lagrange_node(b.res, ip[0], ip[1], ip[2], j)) != TF(0);
-  }
-  if (!any && !dense) {
-    bnd.w = TF(0);
-    return;
+      for (int j = 0; j < 32; ++j)
+        any |= __ldg(b.vol + lagrange_node(b.res, ip[0], ip[1], ip[2], j)) != TF(0);
+    }
+    if (!any) {
+      bnd.w = TF(0);
+      return;
+    }
   }
   if (b.use_grid) {
     if (inside) {
