@@ -230,11 +230,11 @@ __device__ __forceinline__ TF band_slack(const Cn<TF>& c, const BodyDev<TF>& b, 
 }
 
 // The integrand of the volume map at signed distance dm: 1 inside, W(dm) /
-// W(0) outside (dist_cubic_kernel with 1 / h and k / W(0) rounded once).
+// W(0) outside (dist_cubic_kernel with k / W(0) rounded once).
 template <class TF>
-__device__ __forceinline__ TF extension(TF dm, TF inv_h, TF k_w0) {
+__device__ __forceinline__ TF extension(const Cn<TF>& c, TF dm, TF k_w0) {
   if (dm <= TF(0)) return TF(1);
-  const TF q = dm * inv_h, conj = TF(1) - q;
+  const TF q = over_h(c, dm), conj = TF(1) - q;
   const TF s = q <= TF(0.5) ? (TF(6) * q - TF(6)) * q * q + TF(1)
                             : (q <= TF(1) ? TF(2) * conj * conj * conj : TF(0));
   return s * k_w0;
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(256)
           dist = interpolate_grid(b, b.dist, p);
         else
           dist = shape_sdf(b, p);
-        sum += pt.wd[j * peirce::kNumR + k] * double(extension(dist * b.sign, c.inv_h, k_w0));
+        sum += pt.wd[j * peirce::kNumR + k] * double(extension(c, dist * b.sign, k_w0));
       }
     }
   }

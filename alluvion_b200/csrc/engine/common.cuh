@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
+
 #include "alluvion_b200.h"
 
 namespace alb {
@@ -155,6 +157,7 @@ struct Cn {
   TF h, h2, k, l, w0, radius, vol, mass, rho0, visc, bvisc, eps;
   vec3<TF> g;
   TF inv_h, inv_h2;  // 1 / h and 1 / h^2, rounded once on the host
+  TF inv_h_lo, inv_h2_lo;  // what that rounding left out (over_h)
   // periodic in y (the solvers' step<1>): Const::wrap_length and its
   // half-range bounds (constants.hpp:130-136); wrap = 0 otherwise
   TF wrap_len = 0, wrap_min = 0, wrap_max = 0;
@@ -212,6 +215,8 @@ inline Cn<TF> to_cn(const C& c) {
   o.g = vec3<TF>{c.gravity[0], c.gravity[1], c.gravity[2]};
   o.inv_h = TF(1) / o.h;
   o.inv_h2 = TF(1) / o.h2;
+  o.inv_h_lo = std::fma(-o.h, o.inv_h, TF(1)) * o.inv_h;
+  o.inv_h2_lo = std::fma(-o.h2, o.inv_h2, TF(1)) * o.inv_h2;
   return o;
 }
 
@@ -249,11 +254,26 @@ __device__ __forceinline__ TF W_dist(const Cn<TF>& c, TF r) {
   return s * c.k;
 }
 
+// a / h and a / h^2 as the IEEE quotients but for rare last bits: division by a
+// constant with its reciprocal in two parts (Brisebarre, Muller and Raina,
+// "Accelerating correctly rounded floating-point division when the divisor is
+// known in advance", 2004).
+__device__ __forceinline__ float fma_(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_(double a, double b, double c) { return fma(a, b, c); }
+template <class TF>
+__device__ __forceinline__ TF over_h(const Cn<TF>& c, TF a) {
+  return fma_(a, c.inv_h, a * c.inv_h_lo);
+}
+template <class TF>
+__device__ __forceinline__ TF over_h2(const Cn<TF>& c, TF a) {
+  return fma_(a, c.inv_h2, a * c.inv_h2_lo);
+}
+
 // Cubic spline of a squared distance (d2_cubic_kernel, runner.hpp:608-619).
 // float: q from the hardware reciprocal square root and 1/h, no IEEE
 // division or square-root sequence (the reference is built with
 // --use_fast_math, whose division and sqrt are approximate as well).  double:
-// one rsqrt (within one ulp) and 1/h instead of a square root and two divisions.
+// the square root and the quotients as rounded by IEEE operations.
 __device__ __forceinline__ float W_r2(const Cn<float>& c, float r2) {
   const float q2 = r2 * c.inv_h2;
   const float q = r2 > 0.f ? r2 * rsqrtf(r2) * c.inv_h : 0.f;
@@ -266,8 +286,8 @@ __device__ __forceinline__ float W_r2(const Cn<float>& c, float r2) {
   return s * c.k;
 }
 __device__ __forceinline__ double W_r2(const Cn<double>& c, double r2) {
-  const double q2 = r2 * c.inv_h2;
-  const double q = r2 > 0. ? r2 * rsqrt(r2) * c.inv_h : 0.;
+  const double q2 = over_h2(c, r2);
+  const double q = over_h(c, sqrt(r2));
   const double conj = 1. - q;
   double s = 0.;
   if (q <= 0.5)
@@ -278,17 +298,28 @@ __device__ __forceinline__ double W_r2(const Cn<double>& c, double r2) {
 }
 
 // Kernel gradient of a displacement (displacement_cubic_kernel_grad,
-// runner.hpp:628-638): one reciprocal square root gives both |d| and 1/|d|.
-// Double, 127,041 particles: step 846 -> 694 us against a square root and
-// three divisions.
-template <class TF>
-__device__ __forceinline__ vec3<TF> gradW(const Cn<TF>& c, vec3<TF> d) {
-  const TF rl2 = length_sqr(d);
-  const TF inv_rl = rl2 > TF(0) ? rsqrt_(rl2) : TF(0);
-  const TF rl = rl2 * inv_rl;
-  const TF q = rl * c.inv_h;
-  const TF s = q <= TF(0.5) ? (q * TF(3) - TF(2)) * c.inv_h
-                            : (q <= TF(1) ? (TF(1) - q) * (q - TF(1)) * inv_rl : TF(0));
+// runner.hpp:628-638).  float: one hardware reciprocal square root gives
+// both |d| and 1/|d|.
+__device__ __forceinline__ vec3<float> gradW(const Cn<float>& c, vec3<float> d) {
+  const float rl2 = length_sqr(d);
+  const float inv_rl = rl2 > 0.f ? rsqrtf(rl2) : 0.f;
+  const float rl = rl2 * inv_rl;
+  const float q = rl * c.inv_h;
+  const float s = q <= 0.5f ? (q * 3.f - 2.f) * c.inv_h
+                            : (q <= 1.f ? (1.f - q) * (q - 1.f) * inv_rl : 0.f);
+  return (c.l * s) * d;
+}
+// double: no division.  Sums of it against 80-bit ones, over seven radii: 2.98e-16
+// off; 3.07e-16 with its three divisions; 3.20e-16 with |d| by rsqrt and 1/h
+// rounded once (densities 1.70e-16, 1.70e-16, 1.81e-16; a DFSPH step's velocities
+// 1.80e-14, 1.80e-14, 1.93e-14).  The step of 127,041 particles takes 731, 827 and
+// 700 us.
+__device__ __forceinline__ vec3<double> gradW(const Cn<double>& c, vec3<double> d) {
+  const double rl2 = length_sqr(d);
+  const double inv_rl = rl2 > 0. ? rsqrt(rl2) : 0.;
+  const double q = over_h(c, sqrt(rl2));
+  const double s = q <= 0.5 ? over_h(c, q * 3. - 2.)
+                            : (q <= 1. ? (1. - q) * (q - 1.) * inv_rl : 0.);
   return (c.l * s) * d;
 }
 
