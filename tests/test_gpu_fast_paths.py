@@ -1,6 +1,7 @@
 """Edges of the step's and the sampling's kernels: list groups and packed
-distance tests at ragged sizes, the two forms of the cell scan, chunks of
-samples, solver loops of no iteration or several, unaligned list rows."""
+distance tests at ragged sizes, the two forms of the cell scan, large sample
+capacities, solver loops of no iteration or several, unaligned list rows, the
+boundary stop."""
 import ctypes
 
 import numpy as np
